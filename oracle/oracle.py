@@ -356,8 +356,10 @@ class RefLib:
 
     @staticmethod
     def available() -> bool:
-        return REF_SO.exists() or (HERE / "_ref" / "src" / "amips_slice.inc").exists() or \
-            (_recipe().reference_root() / "src").is_dir()
+        if REF_SO.exists() or (HERE / "_ref" / "src" / "amips_slice.inc").exists():
+            return True
+        root = _recipe().reference_root()   # None: no checkout named
+        return root is not None and (root / "src").is_dir()
 
     def amips_batch_soa(self, T, nthreads=1, energy=True, jacobian=True, hessian=True):
         T = _c(T, np.float64)
