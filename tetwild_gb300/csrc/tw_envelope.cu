@@ -1260,77 +1260,98 @@ __device__ __forceinline__ int trunc_int(double x) {
     return (int)x;
 }
 
-// The per-face constants of sampleTriangle.
+// The per-face constants of sampleTriangle.  The face's vertices from the
+// longest edge on (v0, v1 its ends) are kept apart (FaceVerts): the kernels
+// read them from the face itself.  The edge directions are n01, n12 (v1->v2)
+// and -n02 (v2->v0).
+struct FaceVerts {
+    V3 v0, v1, v2;
+};
 struct SampleHeader {
-    V3 vs[3];
-    V3 v0, v1, v2, n01, n02, n12;
-    double ls[3];
-    int max_i;
+    V3 n01, n02, n12;
     double N;           // base-row bound after the N == int(N) adjustment
-    int trivial;        // N <= 1: the three vertices only
-    int M;              // number of candidate rows (M < 1: base row, v1, v2 only)
     double sin_v0, tan_v0, sin_v1;
     double NE, NF;      // edge bounds after the N == int(N) adjustment
-    int hasE, hasF;     // the reference samples an edge only when its raw N > 1
-    V3 nE, nF;          // edge directions v1->v2, v2->v0
+    int max_i;          // v0 is the face's vertex max_i
+    int trivial;        // N <= 1: the three vertices only
+    int M;              // number of candidate rows (M < 1: base row, v1, v2 only)
+    int8_t hasE, hasF;  // the reference samples an edge only when its raw N > 1
+    // sample spacing along v0->v1, v1->v2, v2->v0 and row spacing, each in
+    // units of the edge (the row's: of v0->v2)
+    float r01, r12, r20, rrow;
 };
 
-__device__ __forceinline__ void sample_header(const double* t, double sd, SampleHeader& h) {
-    const double sqrt3_2 = sqrt(3.0) / 2.0;
-    h.vs[0] = V3{t[0], t[1], t[2]};
-    h.vs[1] = V3{t[3], t[4], t[5]};
-    h.vs[2] = V3{t[6], t[7], t[8]};
-    for (int i = 0; i < 3; ++i) h.ls[i] = vlen2(vsub(h.vs[i], h.vs[(i + 1) % 3]));
-    int max_i = 0;
-    for (int i = 1; i < 3; ++i)
-        if (!(h.ls[i] < h.ls[max_i])) max_i = i;
-    h.max_i = max_i;
-    double N = sqrt(h.ls[max_i]) / sd;
-    h.trivial = (N <= 1) ? 1 : 0;
-    h.M = 0;
-    if (h.trivial) return;
-    if (N == (double)trunc_int(N)) N -= 1;
-    h.N = N;
-    h.v0 = h.vs[max_i];
-    h.v1 = h.vs[(max_i + 1) % 3];
-    h.v2 = h.vs[(max_i + 2) % 3];
-    h.n01 = vnormalize(vsub(h.v1, h.v0));
-    double hh = vdist(vadd(vdiv(smul(dot3(vsub(h.v2, h.v0), vsub(h.v1, h.v0)), vsub(h.v1, h.v0)),
-                               h.ls[max_i]),
-                          h.v0),
-                     h.v2);
-    h.M = trunc_int(hh / (sqrt3_2 * sd));
-    if (h.M < 1) return;
-    h.n02 = vnormalize(vsub(h.v2, h.v0));
-    h.n12 = vnormalize(vsub(h.v2, h.v1));
-    double cr0 = vlen(cross3(vsub(h.v2, h.v0), vsub(h.v1, h.v0)));
-    double cr1 = vlen(cross3(vsub(h.v2, h.v1), vsub(h.v0, h.v1)));
-    h.sin_v0 = cr0 / (vdist(h.v0, h.v2) * vdist(h.v0, h.v1));
-    h.tan_v0 = cr0 / dot3(vsub(h.v2, h.v0), vsub(h.v1, h.v0));
-    h.sin_v1 = cr1 / (vdist(h.v1, h.v2) * vdist(h.v0, h.v1));
-    double NE = sqrt(h.ls[(max_i + 1) % 3]) / sd;
-    h.hasE = NE > 1;
-    if (h.hasE && NE == (double)trunc_int(NE)) NE -= 1;
-    h.NE = NE;
-    h.nE = vnormalize(vsub(h.v2, h.v1));
-    double NF = sqrt(h.ls[(max_i + 2) % 3]) / sd;
-    h.hasF = NF > 1;
-    if (h.hasF && NF == (double)trunc_int(NF)) NF -= 1;
-    h.NF = NF;
-    h.nF = vnormalize(vsub(h.v0, h.v2));
+__device__ __forceinline__ FaceVerts face_verts(const double* t, int max_i) {
+    const V3 a{t[0], t[1], t[2]}, b{t[3], t[4], t[5]}, c{t[6], t[7], t[8]};
+    return max_i == 0 ? FaceVerts{a, b, c} : max_i == 1 ? FaceVerts{b, c, a} : FaceVerts{c, a, b};
 }
 
-// Row m (1 <= m <= M): start point v and last index N1; returns false when
-// the row triggers the reference's break (distance(v0_m, v1_m) <= sd).
-__device__ __forceinline__ bool sample_row(const SampleHeader& h, double sd, int m, V3& v, int& N1) {
+__device__ __forceinline__ void sample_header(const double* t, double sd, SampleHeader& h,
+                                              FaceVerts& v) {
+    const double sqrt3_2 = sqrt(3.0) / 2.0;
+    const V3 a{t[0], t[1], t[2]}, b{t[3], t[4], t[5]}, c{t[6], t[7], t[8]};
+    const double lab = vlen2(vsub(a, b)), lbc = vlen2(vsub(b, c)), lca = vlen2(vsub(c, a));
+    int max_i = 0;
+    double l01 = lab, l12 = lbc, l20 = lca;
+    if (!(lbc < l01)) {
+        max_i = 1;
+        l01 = lbc; l12 = lca; l20 = lab;
+    }
+    if (!(lca < l01)) {
+        max_i = 2;
+        l01 = lca; l12 = lab; l20 = lbc;
+    }
+    h.max_i = max_i;
+    v = face_verts(t, max_i);
+    double N = sqrt(l01) / sd;
+    h.trivial = (N <= 1) ? 1 : 0;
+    h.M = 0;
+    h.r01 = h.r12 = h.r20 = h.rrow = 0.0f;
+    if (h.trivial) return;
+    h.r01 = 1.0f / d2f_rn(N);
+    if (N == (double)trunc_int(N)) N -= 1;
+    h.N = N;
+    h.n01 = vnormalize(vsub(v.v1, v.v0));
+    double hh = vdist(vadd(vdiv(smul(dot3(vsub(v.v2, v.v0), vsub(v.v1, v.v0)), vsub(v.v1, v.v0)),
+                               l01),
+                          v.v0),
+                     v.v2);
+    h.M = trunc_int(hh / (sqrt3_2 * sd));
+    if (h.M < 1) return;
+    h.n02 = vnormalize(vsub(v.v2, v.v0));
+    h.n12 = vnormalize(vsub(v.v2, v.v1));
+    double cr0 = vlen(cross3(vsub(v.v2, v.v0), vsub(v.v1, v.v0)));
+    double cr1 = vlen(cross3(vsub(v.v2, v.v1), vsub(v.v0, v.v1)));
+    const double d02 = vdist(v.v0, v.v2), d01 = vdist(v.v0, v.v1);
+    h.sin_v0 = cr0 / (d02 * d01);
+    h.tan_v0 = cr0 / dot3(vsub(v.v2, v.v0), vsub(v.v1, v.v0));
+    h.sin_v1 = cr1 / (vdist(v.v1, v.v2) * d01);
+    h.rrow = d2f_rn(sqrt3_2 * sd) / (d2f_rn(h.sin_v0) * d2f_rn(d02));
+    double NE = sqrt(l12) / sd;
+    h.hasE = NE > 1;
+    h.r12 = 1.0f / d2f_rn(NE);
+    if (h.hasE && NE == (double)trunc_int(NE)) NE -= 1;
+    h.NE = NE;
+    double NF = sqrt(l20) / sd;
+    h.hasF = NF > 1;
+    h.r20 = 1.0f / d2f_rn(NF);
+    if (h.hasF && NF == (double)trunc_int(NF)) NF -= 1;
+    h.NF = NF;
+}
+
+// Row m (1 <= m <= M): start point v, its distance delta_d from the edge
+// v0->v2 and last index N1; returns false when the row triggers the
+// reference's break (distance(v0_m, v1_m) <= sd).
+__device__ __forceinline__ bool sample_row(const SampleHeader& h, const FaceVerts& f, double sd,
+                                           int m, V3& v, int& N1, double& delta_d) {
     const double sqrt3_2 = sqrt(3.0) / 2.0;
     int n = trunc_int(sqrt3_2 / h.tan_v0 * m + 0.5);
     int n1 = trunc_int(sqrt3_2 / h.tan_v0 * m);
     if (m % 2 == 0 && n == n1) n += 1;
-    V3 v0_m = vadd(h.v0, smul((double)m * sqrt3_2 * sd / h.sin_v0, h.n02));
-    V3 v1_m = vadd(h.v1, smul((double)m * sqrt3_2 * sd / h.sin_v1, h.n12));
+    V3 v0_m = vadd(f.v0, smul((double)m * sqrt3_2 * sd / h.sin_v0, h.n02));
+    V3 v1_m = vadd(f.v1, smul((double)m * sqrt3_2 * sd / h.sin_v1, h.n12));
     if (vdist(v0_m, v1_m) <= sd) return false;
-    double delta_d = (((double)n + (m % 2) / 2.0) - (double)m * sqrt3_2 / h.tan_v0) * sd;
+    delta_d = (((double)n + (m % 2) / 2.0) - (double)m * sqrt3_2 / h.tan_v0) * sd;
     v = vadd(v0_m, smul(delta_d, h.n01));
     N1 = trunc_int(vdist(v, v1_m) / sd);
     return true;
@@ -1338,12 +1359,14 @@ __device__ __forceinline__ bool sample_row(const SampleHeader& h, double sd, int
 __device__ __forceinline__ V3 row_point(const SampleHeader& h, const V3& v, double sd, int i) {
     return vadd(v, vmul(smul((double)i, h.n01), sd));
 }
-__device__ __forceinline__ V3 base_point(const SampleHeader& h, double sd, int n) {
-    return vadd(h.v0, vmul(vmul(h.n01, sd), (double)n));
+__device__ __forceinline__ V3 base_point(const SampleHeader& h, const FaceVerts& f, double sd,
+                                         int n) {
+    return vadd(f.v0, vmul(vmul(h.n01, sd), (double)n));
 }
 __device__ __forceinline__ V3 edge_point(const V3& o, const V3& dir, double sd, int n) {
     return vadd(o, vmul(vmul(dir, sd), (double)n));
 }
+__device__ __forceinline__ V3 vneg(const V3& a) { return V3{-a.x, -a.y, -a.z}; }
 // number of integers n with lo <= n <= N (N a double), lo >= 0
 __device__ __forceinline__ int count_upto(double N, int lo) {
     if (!(N >= (double)lo)) return 0;
@@ -1440,151 +1463,207 @@ __device__ __forceinline__ void face_query_box(const double* t, const FaceCtx& F
     }
 }
 
-// The samples of one face with its header already computed, the whole warp:
-// 1 if some sample is out, 0 otherwise.
-template <bool FP32>
-__device__ __forceinline__ uint8_t env_face_samples(const SampleHeader& h, const FaceCtx& F,
-                                                    double sd, TravStats& st, uint32_t& nq) {
-    const int lane = threadIdx.x & 31;
-    {
-        int32_t hint = -1;
-        bool out_found = false;
-        // certified mode: the leaves within reach of the face, shared by the
-        // warp (see k_env_points_warp); -1 when above 32 (per-sample walks)
-        int32_t cand = -1;
-        int cnt = -1, kh = 0;
-        if (FP32 && !F.T.gslot) {
-            float qlo[3], qhi[3];
-            const double t[9] = {h.vs[0].x, h.vs[0].y, h.vs[0].z, h.vs[1].x, h.vs[1].y,
-                                 h.vs[1].z, h.vs[2].x, h.vs[2].y, h.vs[2].z};
-            face_query_box(t, F, qlo, qhi);
-            cnt = warp_candidates32(F.T, qlo, qhi, lane, cand);
-            if (cnt == kTraversalError) {
-                if (lane == 0) atomicOr(F.counters + kCntError, 1ULL);
-                cnt = -1;
-            }
+#include "tw_hull.cuh"
 
+// The samples of one face with its header already computed, the whole warp:
+// 1 if some sample is out, 0 otherwise.  Samples in a cut known to be inside
+// (hull) are passed over; the others collect in the warp's queue (64 words of
+// shared memory) and are built and tested 32 at a time, so that the binary64
+// construction and the facet tests run on full warps.  slice / slices: the
+// warp takes every slices-th step of 32 samples; stop (shared, may be null):
+// set by another warp of the face that found a sample out.  Out of line: the
+// sampling kernel calls it from two places.
+template <bool FP32>
+__device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
+                                                    const double* __restrict__ tri,
+                                                    const FaceCuts& hull, int k2, uint32_t* queue,
+                                                    const FaceCtx& F, double sd, int slice,
+                                                    int slices, const volatile int* stop,
+                                                    TravStats& st, uint32_t& nq) {
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    double tv[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) tv[k] = __ldg(tri + k);
+    const FaceVerts fv = face_verts(tv, h.max_i);
+    int32_t hint = -1;
+    // certified mode without a grid: the leaves within reach of the face, shared
+    // by the warp (see k_env_points_warp); -1 when above 32 (per-sample walks)
+    int32_t cand = -1;
+    int cnt = -1, kh = 0;
+    if (FP32 && !F.T.gslot) {
+        float qlo[3], qhi[3];
+        face_query_box(tv, F, qlo, qhi);
+        cnt = warp_candidates32(F.T, qlo, qhi, lane, cand);
+        if (cnt == kTraversalError) {
+            if (lane == 0) atomicOr(F.counters + kCntError, 1ULL);
+            cnt = -1;
         }
-        // out iff the lane's sample (have) is out; called by the whole warp
-        auto lane_out = [&](bool have, const V3& p) -> bool {
-            if (F.T.gslot) {
-                CertQuery q;
-                if (have) q = cert_query(p, F.E, F.T.scale_hi);
-                return have && !grid_point_in<FP32>(F.T, F.E, have, p, q, st);
-            }
-            if (cnt < 0) {
-                bool o = false;
-                if (have) o = sample_out<FP32>(F, p, hint, st);
-                return o;
-            }
-            bool in = !have;
+    }
+    // out iff the lane's sample (have) is out; called by the whole warp
+    auto lane_out = [&](bool have, const V3& p) -> bool {
+        if (F.T.gslot) {
             CertQuery q;
             if (have) q = cert_query(p, F.E, F.T.scale_hi);
-            for (int k = 0; k < cnt; ++k) {
-                const int kk = (k + kh) % cnt;
-                const int32_t lf = __shfl_sync(0xffffffffu, cand, kk);
-                if (!in && cert_leaf_within(F.T.cull, F.T.tri, lf, p, q, F.E.eps2, st)) {
-                    in = true;
-                    kh = kk;
-                }
-                if (__all_sync(0xffffffffu, in)) break;
-            }
-            return !in;
-        };
-        if (h.trivial) {
-            const bool have = lane < 3;
-            out_found = lane_out(have, have ? h.vs[lane] : h.vs[0]);
-            if (have) ++nq;
-            out_found = __any_sync(0xffffffffu, out_found);
-            return out_found ? 1 : 0;
+            return have && !grid_point_in<FP32>(F.T, F.E, have, p, q, st);
         }
-        // The samples as flat index ranges that the 32 lanes walk in step (the
-        // order of the tests changes only the work: the face is out iff some
-        // sample is).  First the base row, v1, v2 and the two other edges...
-        const int NA = count_upto(h.N, 0);
-        const int NE = (h.M >= 1 && h.hasE) ? count_upto(h.NE, 1) : 0;
-        const int NF = (h.M >= 1 && h.hasF) ? count_upto(h.NF, 1) : 0;
-        const int NX = NA + 2 + NE + NF;
-        for (int s0 = 0; s0 < NX; s0 += 32) {
-            const int s = s0 + lane;
-            const bool have = s < NX;
-            V3 p{0.0, 0.0, 0.0};
-            if (have) {
-                if (s < NA) p = base_point(h, sd, s);
-                else if (s == NA) p = h.v1;
-                else if (s == NA + 1) p = h.v2;
-                else if (s < NA + 2 + NE) p = edge_point(h.v1, h.nE, sd, s - NA - 1);
-                else p = edge_point(h.v2, h.nF, sd, s - NA - 1 - NE);
+        if (cnt < 0) {
+            bool o = false;
+            if (have) o = sample_out<FP32>(F, p, hint, st);
+            return o;
+        }
+        bool in = !have;
+        CertQuery q;
+        if (have) q = cert_query(p, F.E, F.T.scale_hi);
+        for (int k = 0; k < cnt; ++k) {
+            const int kk = (k + kh) % cnt;
+            const int32_t lf = __shfl_sync(0xffffffffu, cand, kk);
+            if (!in && cert_leaf_within(F.T.cull, F.T.tri, lf, p, q, F.E.eps2, st)) {
+                in = true;
+                kh = kk;
             }
+            if (__all_sync(0xffffffffu, in)) break;
+        }
+        return !in;
+    };
+    // passed over: the sample at v0 + s (v1 - v0) + t (v2 - v0)
+    auto inside = [&](float s, float t) -> bool {
+        const float r = (1.0f - s) - t;
+        return h.max_i == 0   ? hull_inside(hull, k2, s, t)
+               : h.max_i == 1 ? hull_inside(hull, k2, r, s)
+                              : hull_inside(hull, k2, t, r);
+    };
+    int qn = 0;
+    // tests queued samples in full warps (all: to the last); true when one is out
+    auto drain = [&](bool all, auto&& point) -> bool {
+        while (qn >= 32 || (all && qn > 0)) {
+            const int m = min(qn, 32);
+            qn -= m;
+            const bool have = lane < m;
+            const uint32_t e = have ? queue[qn + lane] : 0u;
+            const V3 p = point(have, e);
             const bool o = lane_out(have, p);
             if (have) ++nq;
-            if (__any_sync(0xffffffffu, o)) return 1;
+            if (__any_sync(0xffffffffu, o || (stop && *stop))) return true;
         }
-        // ...then the rows 1..M, 32 at a time: each lane sets up one row
-        // (start point and last index), the reference's break (the first row
-        // with distance(v0_m, v1_m) <= sd) ends the rows, and the lanes walk
-        // the chunk's samples by flat index.
-        for (int base = 1; base <= h.M; base += 32) {
-            const int m = base + lane;
-            V3 v{0.0, 0.0, 0.0};
-            int N1 = -1;
-            const bool valid = m <= h.M;
-            const bool brk = valid && !sample_row(h, sd, m, v, N1);
-            const unsigned bal = __ballot_sync(0xffffffffu, brk);
-            const int first_brk = bal ? __ffs(bal) - 1 : 32;
-            int cnt = 0;
-            if (valid && lane < first_brk) {
-                if (N1 > (int)kMaxSamplesPerRow) {
-                    atomicOr(F.counters + kCntError, 2ULL);
-                } else {
-                    cnt = N1 + 1;
-                }
-            }
-            int incl = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += t;
-            }
-            const int excl = incl - cnt;
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            for (int s0 = 0; s0 < total; s0 += 32) {
-                const int s = s0 + lane;
-                const bool have = s < total;
-                // the row holding flat index s: the last lane whose first index is
-                // <= s (first indices never decrease; empty rows share the next one's)
-                int r = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int c = r + step;
-                    const int ex = __shfl_sync(0xffffffffu, excl, c & 31);
-                    if (c < 32 && ex <= s) r = c;
-                }
-                const double vx = __shfl_sync(0xffffffffu, v.x, r);
-                const double vy = __shfl_sync(0xffffffffu, v.y, r);
-                const double vz = __shfl_sync(0xffffffffu, v.z, r);
-                const int ex = __shfl_sync(0xffffffffu, excl, r);
-                V3 p{0.0, 0.0, 0.0};
-                if (have) p = row_point(h, V3{vx, vy, vz}, sd, s - ex);
-                const bool o = lane_out(have, p);
-                if (have) ++nq;
-                if (__any_sync(0xffffffffu, o)) return 1;
-            }
-            if (bal) break;
-        }
-        return out_found ? 1 : 0;
+        return false;
+    };
+    auto push = [&](bool want, uint32_t e) {
+        const unsigned bal = __ballot_sync(0xffffffffu, want);
+        if (want) queue[qn + __popc(bal & lt)] = e;
+        qn += __popc(bal);
+        __syncwarp();
+    };
+    if (h.trivial) {
+        const bool have = lane < 3;
+        const bool o = lane_out(have, lane == 1 ? fv.v1 : lane == 2 ? fv.v2 : fv.v0);
+        if (have) ++nq;
+        return __any_sync(0xffffffffu, o) ? 1 : 0;
     }
+    // The samples as flat index ranges that the 32 lanes walk in step (the
+    // order of the tests changes only the work: the face is out iff some
+    // sample is).  First the base row, v1, v2 and the two other edges...
+    const int NA = count_upto(h.N, 0);
+    const int NE = (h.M >= 1 && h.hasE) ? count_upto(h.NE, 1) : 0;
+    const int NF = (h.M >= 1 && h.hasF) ? count_upto(h.NF, 1) : 0;
+    const int NX = NA + 2 + NE + NF;
+    auto rim = [&](bool have, uint32_t e) -> V3 {
+        const int s = (int)e;
+        if (!have) return fv.v0;
+        if (s < NA) return base_point(h, fv, sd, s);
+        if (s == NA) return fv.v1;
+        if (s == NA + 1) return fv.v2;
+        if (s < NA + 2 + NE) return edge_point(fv.v1, h.n12, sd, s - NA - 1);
+        return edge_point(fv.v2, vneg(h.n02), sd, s - NA - 1 - NE);
+    };
+    for (int s0 = 32 * slice; s0 < NX; s0 += 32 * slices) {
+        const int s = s0 + lane;
+        float x, y;   // the sample along v0->v1 and v0->v2
+        if (s < NA) {
+            x = (float)s * h.r01;
+            y = 0.0f;
+        } else if (s < NA + 2) {
+            y = (float)(s - NA);
+            x = 1.0f - y;
+        } else if (s < NA + 2 + NE) {
+            y = (float)(s - NA - 1) * h.r12;
+            x = 1.0f - y;
+        } else {
+            x = 0.0f;
+            y = 1.0f - (float)(s - NA - 1 - NE) * h.r20;
+        }
+        push(s < NX && !inside(x, y), (uint32_t)s);
+        if (drain(false, rim)) return 1;
+    }
+    if (drain(true, rim)) return 1;
+    // ...then the rows 1..M, 32 at a time: each lane sets up one row (start
+    // point and last index), the reference's break (the first row with
+    // distance(v0_m, v1_m) <= sd) ends the rows, and the lanes walk the chunk's
+    // samples by flat index.
+    for (int base = 1; base <= h.M; base += 32) {
+        const int m = base + lane;
+        V3 v{0.0, 0.0, 0.0};
+        int N1 = -1;
+        double dd = 0.0;
+        const bool valid = m <= h.M;
+        const bool brk = valid && !sample_row(h, fv, sd, m, v, N1, dd);
+        const unsigned bal = __ballot_sync(0xffffffffu, brk);
+        const int first_brk = bal ? __ffs(bal) - 1 : 32;
+        int rows = 0;
+        if (valid && lane < first_brk) {
+            if (N1 > (int)kMaxSamplesPerRow) {
+                atomicOr(F.counters + kCntError, 2ULL);
+            } else {
+                rows = N1 + 1;
+            }
+        }
+        // the row's first sample along v0->v1: delta_d in units of the edge
+        const float sx = d2f_rn(dd) / d2f_rn(sd) * h.r01;
+        int incl = rows;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        const int excl = incl - rows;
+        const int total = __shfl_sync(0xffffffffu, incl, 31);
+        auto in_row = [&](bool, uint32_t e) -> V3 {   // e: row << 26 | index (below 2^23)
+            const int r = (int)(e >> 26);
+            const V3 w{__shfl_sync(0xffffffffu, v.x, r), __shfl_sync(0xffffffffu, v.y, r),
+                       __shfl_sync(0xffffffffu, v.z, r)};
+            return row_point(h, w, sd, (int)(e & 0x3ffffffu));
+        };
+        for (int s0 = 32 * slice; s0 < total; s0 += 32 * slices) {
+            const int s = s0 + lane;
+            // the row holding flat index s: the last lane whose first index is
+            // <= s (first indices never decrease; empty rows share the next one's)
+            int r = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1) {
+                const int c = r + step;
+                const int ex = __shfl_sync(0xffffffffu, excl, c & 31);
+                if (c < 32 && ex <= s) r = c;
+            }
+            const int i = s - __shfl_sync(0xffffffffu, excl, r);
+            const float x = fmaf((float)i, h.r01, __shfl_sync(0xffffffffu, sx, r));
+            push(s < total && !inside(x, (float)(base + r) * h.rrow),
+                 ((uint32_t)r << 26) | (uint32_t)i);
+            if (drain(false, in_row)) return 1;
+        }
+        if (drain(true, in_row)) return 1;
+        if (bal) break;
+    }
+    return 0;
 }
 
 // Header stage of one face (one thread): 0 = degenerate (not out), 1 = beyond
-// the per-row sample bound (error bit 2, counted out), 2 = sample it.
-__device__ __forceinline__ int face_prepare(const double* __restrict__ tri, double sd,
+// the per-row sample bound (error bit 2, counted out), 2 = sample it.  shaped:
+// known not to be degenerate (hull_prepare).
+__device__ __forceinline__ int face_prepare(const double* t, double sd, bool shaped,
                                             SampleHeader& h, unsigned long long* counters) {
-    double t[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + k);
-    if (tri_collinear(t)) return 0;
-    sample_header(t, sd, h);
+    if (!shaped && tri_collinear(t)) return 0;
+    FaceVerts v;
+    sample_header(t, sd, h, v);
     if (header_too_large(h)) {
         atomicOr(counters + kCntError, 2ULL);
         return 1;
@@ -1592,132 +1671,244 @@ __device__ __forceinline__ int face_prepare(const double* __restrict__ tri, doub
     return 2;
 }
 
-// One face, the whole warp (every lane computes the header).
-template <bool FP32>
-__device__ __forceinline__ uint8_t env_face_warp(const double* __restrict__ tri,
-                                                 const FaceCtx& F, double sd, TravStats& st,
-                                                 uint32_t& nq) {
-    SampleHeader h;
-    double t[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) t[k] = __ldg(tri + k);
-    if (tri_collinear(t)) return 0;
-    sample_header(t, sd, h);
-    if (header_too_large(h)) {
-        if ((threadIdx.x & 31) == 0) atomicOr(F.counters + kCntError, 2ULL);
-        return 1;
-    }
-    return env_face_samples<FP32>(h, F, sd, st, nq);
-}
-
-// Faces in blocks of kFaceBlock: first every thread prepares one face's header
-// into shared memory (the FP64 header and the exact degeneracy test run once
-// per face instead of once per lane), then each warp samples its share of the
-// block's faces.  Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
+// Faces run in two launches.  The first cuts every face, a warp a face, in
+// binary32 only, and answers those that are inside as a whole (0) or have a
+// vertex certainly out (1); the others it marks open (kFaceOpen in out).  The
+// second samples the open faces: their binary64 headers, one a thread, then a
+// face by a warp, which cuts it again, now keeping its open pieces, and tests
+// the samples there.  (In one kernel the cut was held to the 16 warps per SM
+// of the sampling's 128 registers, and half of its stalls were barriers.)
+// Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
+// to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 3.0 and 0.76.
+// Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
+constexpr int kFaceWarps = kFaceBlock / 32;
+constexpr int kCutBlocks = 8, kSampleBlocks = 4;   // blocks per SM
+constexpr uint8_t kFaceOpen = 2;
+// pieces that a sample is worth: its binary64 distance costs that of several
+constexpr float kSampleCost32 = 0.6f, kSampleCost64 = 1.0f;
 
-struct FaceSlot {
-    SampleHeader h;
-    int32_t state;  // face_prepare's result, or -1 past the end
-    int32_t seg;
-};
-
+// A warp takes an eighth of its share of the faces at a time (4 to 32), so
+// that small batches spread over all SMs and large ones balance.
 template <bool FP32, class Ctx>
-__device__ __forceinline__ void faces_blocked(const double* __restrict__ tris, int64_t n,
-                                              unsigned long long* counters, Ctx ctx,
-                                              uint8_t* __restrict__ out) {
-    __shared__ FaceSlot slot[kFaceBlock];
+__device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64_t n,
+                                          unsigned long long* counters, Ctx ctx,
+                                          uint8_t* __restrict__ out) {
+    __shared__ CutTables tab;
+    __shared__ FaceFrame frame[kFaceWarps][32];
+    fill_cut_tables(tab);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
     TravStats st;
-    uint32_t nq = 0;
-    for (int64_t base = (int64_t)blockIdx.x * kFaceBlock; base < n;
-         base += (int64_t)gridDim.x * kFaceBlock) {
-        for (int k = threadIdx.x; k < kFaceBlock; k += blockDim.x) {
-            const int64_t f = base + k;
-            FaceSlot& fs = slot[k];
-            if (f >= n) {
-                fs.state = -1;
-                continue;
-            }
+    uint32_t nq = 0, nopen = 0;
+    const int64_t warps = (int64_t)gridDim.x * kFaceWarps, share = n / (warps * 8);
+    const int tile = (int)(share < 4 ? 4 : share > 32 ? 32 : share);
+    for (int64_t base = ((int64_t)blockIdx.x * kFaceWarps + warp) * tile; base < n;
+         base += warps * tile) {
+        const int faces = (int)(n - base < tile ? n - base : tile);
+        if (lane < faces) {
+            FaceCtx F;
+            double sd, t[9];
+            ctx(base + lane, F, sd);
+#pragma unroll
+            for (int k = 0; k < 9; ++k) t[k] = __ldg(tris + 9 * (base + lane) + k);
+            hull_prepare(t, F.T, F.E, sd, FP32 ? kSampleCost32 : kSampleCost64,
+                         frame[warp][lane]);
+        }
+        __syncwarp();
+        int o = kFaceOpen;
+        for (int k = 0; k < faces; ++k) {
+            const FaceFrame& h = frame[warp][k];
+            if (h.k2 < 0) continue;
             FaceCtx F;
             double sd;
-            fs.seg = ctx(f, F, sd);
-            fs.state = face_prepare(tris + 9 * f, sd, fs.h, counters);
+            ctx(base + k, F, sd);
+            const int r = hull_cut<false>(F.T, F.E, h, tris + 9 * (base + k), tab, nullptr, 0, 1,
+                                          st, nq);
+            if (lane == k) o = r;
         }
+        if (lane < faces) {
+            out[base + lane] = (uint8_t)o;
+            nopen += o == kFaceOpen;
+        }
+        __syncwarp();
+    }
+    nopen = __reduce_add_sync(0xffffffffu, nopen);
+    if (lane == 0 && nopen) atomicAdd(counters + kCntFaceOpen, (unsigned long long)nopen);
+    flush_stats(st, counters, nq);
+}
+
+// Samples of a face from which on the block's warps share it.
+constexpr int kSharedFace = 384;
+
+// The open faces are sparse and their work differs by orders of magnitude
+// (the ideal length against refined edges, samples near a vertex of many
+// facets).  Blocks take ranges of faces from a counter, each long enough to
+// hold about a quarter of a block's share of the open ones (at most one a
+// thread); every thread prepares one of them, the warps take the small ones in
+// turn, and then the four warps share the samples and second cuts of each
+// large one (a launch otherwise lasts as long as its largest face).
+template <bool FP32, class Ctx>
+__device__ __forceinline__ void faces_sample(const double* __restrict__ tris, int64_t n,
+                                             unsigned long long* counters, Ctx ctx,
+                                             uint8_t* __restrict__ out) {
+    __shared__ CutTables tab;
+    __shared__ FaceFrame frame[kFaceBlock];
+    __shared__ SampleHeader head[kFaceBlock];
+    __shared__ FaceCuts cuts[kFaceWarps];
+    __shared__ uint32_t queue[kFaceWarps][64];
+    __shared__ uint16_t list[kFaceBlock];
+    __shared__ uint8_t small[kFaceBlock], large[kFaceBlock];
+    __shared__ int held, nsmall, nlarge, next, found;
+    __shared__ unsigned long long at;
+    const unsigned long long nopen = counters[kCntFaceOpen];
+    if (nopen == 0) return;
+    fill_cut_tables(tab);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    TravStats st;
+    uint32_t nq = 0;
+    const double want = fmin(fmax((double)nopen / (4.0 * gridDim.x), 2.0), (double)kFaceBlock);
+    const int range = (int)fmin(want * ((double)n / (double)nopen), 4096.0) + 1;
+    for (;;) {
+        if (threadIdx.x == 0)
+            at = atomicAdd(counters + kCntFaceNext, (unsigned long long)range);
         __syncthreads();
-        for (int k = warp; k < kFaceBlock; k += nwarps) {
-            const int64_t f = base + k;
-            const FaceSlot& fs = slot[k];
-            if (fs.state < 0) break;
-            uint8_t o = (uint8_t)fs.state;
-            if (fs.state == 2) {
+        const int64_t base = (int64_t)at;
+        if (base >= n) break;
+        const int faces = (int)(n - base < range ? n - base : range);
+        int r0 = 0;
+        while (r0 < faces) {
+            // the next open faces of the range, at most one a thread
+            if (threadIdx.x == 0) held = nsmall = nlarge = next = found = 0;
+            __syncthreads();
+            int before = 0;   // held before this step, the same on every thread
+            while (r0 < faces && before <= kFaceBlock - kFaceBlock / 4) {
+                // a quarter block of flags a step by each warp in turn would idle
+                // the others: all threads read, and stop before the list can overflow
+                const int step = min(kFaceBlock - before, faces - r0);
+                const int f = r0 + threadIdx.x;
+                if ((int)threadIdx.x < step && out[base + f] == kFaceOpen)
+                    list[atomicAdd(&held, 1)] = (uint16_t)f;
+                r0 += step;
+                __syncthreads();
+                before = held;
+                __syncthreads();
+            }
+            const int batch = before;
+            if ((int)threadIdx.x < batch) {
+                const int64_t f = base + list[threadIdx.x];
+                FaceCtx F;
+                double sd, t[9];
+                ctx(f, F, sd);
+#pragma unroll
+                for (int k = 0; k < 9; ++k) t[k] = __ldg(tris + 9 * f + k);
+                hull_prepare(t, F.T, F.E, sd, FP32 ? kSampleCost32 : kSampleCost64,
+                             frame[threadIdx.x]);
+                SampleHeader& h = head[threadIdx.x];
+                const int state = face_prepare(t, sd, frame[threadIdx.x].k2 >= 0, h, counters);
+                if (state != 2) {
+                    out[f] = (uint8_t)state;
+                } else if (!h.trivial && h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace) {
+                    large[atomicAdd(&nlarge, 1)] = (uint8_t)threadIdx.x;
+                } else {
+                    small[atomicAdd(&nsmall, 1)] = (uint8_t)threadIdx.x;
+                }
+            }
+            __syncthreads();
+            for (;;) {
+                int j = 0;
+                if (lane == 0) j = atomicAdd(&next, 1);
+                j = __shfl_sync(0xffffffffu, j, 0);
+                if (j >= nsmall) break;
+                const int k = small[j];
+                const int64_t f = base + list[k];
                 FaceCtx F;
                 double sd;
                 ctx(f, F, sd);
-                o = env_face_samples<FP32>(fs.h, F, sd, st, nq);
+                if (frame[k].k2 >= 0)
+                    hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[warp], 0, 1, st, nq);
+                const uint8_t o =
+                    env_face_samples<FP32>(head[k], tris + 9 * f, cuts[warp], frame[k].k2,
+                                           queue[warp], F, sd, 0, 1, nullptr, st, nq);
+                if (lane == 0) out[f] = o;
+                __syncwarp();
             }
-            if (lane == 0) out[f] = o;
+            for (int j = 0; j < nlarge; ++j) {
+                const int k = large[j];
+                const int64_t f = base + list[k];
+                FaceCtx F;
+                double sd;
+                ctx(f, F, sd);
+                __syncthreads();   // cuts[0] is free, found is 0
+                if (frame[k].k2 >= 0)
+                    hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[0], warp,
+                                   kFaceWarps, st, nq);
+                __syncthreads();
+                if (env_face_samples<FP32>(head[k], tris + 9 * f, cuts[0], frame[k].k2,
+                                           queue[warp], F, sd, warp, kFaceWarps, &found, st, nq))
+                    found = 1;
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    out[f] = (uint8_t)found;
+                    found = 0;
+                }
+            }
+            __syncthreads();
         }
         __syncthreads();
     }
     flush_stats(st, counters, nq);
 }
 
+// All faces with one tree; n_dev (may be null): the count, known only on the
+// device (at most n, for which the grids are sized; warps beyond it exit at once).
+struct OneFaceCtx {
+    FaceCtx F;
+    double sd;
+    __device__ __forceinline__ void operator()(int64_t, FaceCtx& Fo, double& sdo) const {
+        Fo = F;
+        sdo = sd;
+    }
+};
+__device__ __forceinline__ int64_t faces_count(int64_t n, const unsigned long long* n_dev) {
+    return n_dev ? (int64_t)min((unsigned long long)n, *n_dev) : n;
+}
 template <bool FP32>
-__device__ __forceinline__ void k_env_faces_body(const double* __restrict__ tris, int64_t n,
-                                                 const FaceCtx& F, double sd,
-                                                 uint8_t* __restrict__ out) {
-    faces_blocked<FP32>(tris, n, F.counters,
-                        [&](int64_t, FaceCtx& Fo, double& sdo) {
-                            Fo = F;
-                            sdo = sd;
-                            return 0;
-                        },
-                        out);
+__global__ void __launch_bounds__(kFaceBlock, kCutBlocks)
+    k_env_faces_cut(const double* __restrict__ tris, int64_t n,
+                    const unsigned long long* __restrict__ n_dev, OneFaceCtx C,
+                    uint8_t* __restrict__ out) {
+    faces_cut<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, out);
+}
+template <bool FP32>
+__global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
+    k_env_faces(const double* __restrict__ tris, int64_t n,
+                const unsigned long long* __restrict__ n_dev, OneFaceCtx C,
+                uint8_t* __restrict__ out) {
+    faces_sample<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, out);
 }
 
-template <bool FP32>
-__global__ void __launch_bounds__(128, 4) k_env_faces(const double* __restrict__ tris, int64_t n,
-                                                   FaceCtx F, double sd, uint8_t* __restrict__ out) {
-    k_env_faces_body<FP32>(tris, n, F, sd, out);
+// n_dev: nullptr, or the device count of the faces (at most n)
+void launch_env_faces_dev(const Surface& S, const double* tris, const unsigned long long* n_dev,
+                          int64_t n, double eps2, double sd, uint8_t* out, int precision,
+                          unsigned long long* counters, cudaStream_t s) {
+    if (n <= 0) return;
+    const int block = kFaceBlock;
+    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
+    cudaMemsetAsync(counters + kCntFaceOpen, 0, 2 * sizeof(unsigned long long), s);
+    const OneFaceCtx C{FaceCtx{env_tree_for(S, eps2), eps_params(eps2), counters}, sd};
+    if (precision == TW_PRECISION_FP32_CERTIFIED) {
+        k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<true><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
+    } else {
+        k_env_faces_cut<false><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<false><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
+    }
 }
 
 void launch_env_faces(const Surface& S, const double* tris, int64_t n, double eps2, double sd,
                       uint8_t* out, int precision, unsigned long long* counters, cudaStream_t s) {
-    if (n <= 0) return;
-    const int block = kFaceBlock;
-    int grid = grid_for(n, block, 4);
-    FaceCtx F{env_tree_for(S, eps2), eps_params(eps2), counters};
-    if (precision == TW_PRECISION_FP32_CERTIFIED) {
-        k_env_faces<true><<<grid, block, 0, s>>>(tris, n, F, sd, out);
-    } else {
-        k_env_faces<false><<<grid, block, 0, s>>>(tris, n, F, sd, out);
-    }
-}
-
-// Envelope faces whose count is known only on the device (*n_dev, at most
-// cap): the grid is sized for cap and the warps beyond *n_dev exit at once.
-template <bool FP32>
-__global__ void __launch_bounds__(128, 4) k_env_faces_dev(const double* __restrict__ tris,
-                                                       const unsigned long long* __restrict__ n_dev,
-                                                       int64_t cap, FaceCtx F, double sd,
-                                                       uint8_t* __restrict__ out) {
-    const int64_t n = (int64_t)min((unsigned long long)cap, *n_dev);
-    k_env_faces_body<FP32>(tris, n, F, sd, out);
-}
-
-void launch_env_faces_dev(const Surface& S, const double* tris, const unsigned long long* n_dev,
-                          int64_t cap, double eps2, double sd, uint8_t* out, int precision,
-                          unsigned long long* counters, cudaStream_t s) {
-    if (cap <= 0) return;
-    const int block = kFaceBlock;
-    int grid = grid_for(cap, block, 4);
-    FaceCtx F{env_tree_for(S, eps2), eps_params(eps2), counters};
-    if (precision == TW_PRECISION_FP32_CERTIFIED)
-        k_env_faces_dev<true><<<grid, block, 0, s>>>(tris, n_dev, cap, F, sd, out);
-    else
-        k_env_faces_dev<false><<<grid, block, 0, s>>>(tris, n_dev, cap, F, sd, out);
+    launch_env_faces_dev(S, tris, nullptr, n, eps2, sd, out, precision, counters, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1783,20 +1974,27 @@ __global__ void __launch_bounds__(128) k_env_points_segs(const double* __restric
     flush_stats(st, counters, nq);
 }
 
+struct SegFaceCtx {
+    const EnvSeg* segs;
+    int nsegs;
+    unsigned long long* counters;
+    __device__ __forceinline__ void operator()(int64_t f, FaceCtx& Fo, double& sdo) const {
+        const EnvSeg& g = segs[find_seg(segs, nsegs, f)];
+        Fo = FaceCtx{g.T, g.E, counters};
+        sdo = g.sd;
+    }
+};
 template <bool FP32>
-__global__ void __launch_bounds__(128, 4) k_env_faces_segs(const double* __restrict__ tris, int64_t n,
-                                                        const EnvSeg* __restrict__ segs, int nsegs,
-                                                        uint8_t* __restrict__ out,
-                                                        unsigned long long* __restrict__ counters) {
-    faces_blocked<FP32>(tris, n, counters,
-                        [&](int64_t f, FaceCtx& Fo, double& sdo) {
-                            const int k = find_seg(segs, nsegs, f);
-                            const EnvSeg& g = segs[k];
-                            Fo = FaceCtx{g.T, g.E, counters};
-                            sdo = g.sd;
-                            return k;
-                        },
-                        out);
+__global__ void __launch_bounds__(kFaceBlock, kCutBlocks)
+    k_env_faces_segs_cut(const double* __restrict__ tris, int64_t n, SegFaceCtx C,
+                         uint8_t* __restrict__ out) {
+    faces_cut<FP32>(tris, n, C.counters, C, out);
+}
+template <bool FP32>
+__global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
+    k_env_faces_segs(const double* __restrict__ tris, int64_t n, SegFaceCtx C,
+                     uint8_t* __restrict__ out) {
+    faces_sample<FP32>(tris, n, C.counters, C, out);
 }
 
 void launch_env_points_segs(const double* P, int64_t n, const void* segs, int nsegs, uint8_t* out,
@@ -1815,12 +2013,16 @@ void launch_env_faces_segs(const double* tris, int64_t n, const void* segs, int 
                            int precision, unsigned long long* counters, cudaStream_t s) {
     if (n <= 0 || nsegs <= 0) return;
     const int block = kFaceBlock;
-    const int grid = grid_for(n, block, 4);
-    const EnvSeg* g = static_cast<const EnvSeg*>(segs);
-    if (precision == TW_PRECISION_FP32_CERTIFIED)
-        k_env_faces_segs<true><<<grid, block, 0, s>>>(tris, n, g, nsegs, out, counters);
-    else
-        k_env_faces_segs<false><<<grid, block, 0, s>>>(tris, n, g, nsegs, out, counters);
+    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
+    cudaMemsetAsync(counters + kCntFaceOpen, 0, 2 * sizeof(unsigned long long), s);
+    const SegFaceCtx C{static_cast<const EnvSeg*>(segs), nsegs, counters};
+    if (precision == TW_PRECISION_FP32_CERTIFIED) {
+        k_env_faces_segs_cut<true><<<gc, block, 0, s>>>(tris, n, C, out);
+        k_env_faces_segs<true><<<gs, block, 0, s>>>(tris, n, C, out);
+    } else {
+        k_env_faces_segs_cut<false><<<gc, block, 0, s>>>(tris, n, C, out);
+        k_env_faces_segs<false><<<gs, block, 0, s>>>(tris, n, C, out);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2457,15 +2659,14 @@ void launch_smooth_project(const Surface& Sin, const Surface& Sb, double eps2,
 __global__ void k_sample_triangle(const double* __restrict__ t, double sd, double* out,
                                   int64_t cap, int64_t* count) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    {
-        double tv[9];
-        for (int k = 0; k < 9; ++k) tv[k] = t[k];
-        SampleHeader h;
-        sample_header(tv, sd, h);
-        if (header_too_large(h)) {
-            *count = -1;
-            return;
-        }
+    double tv[9];
+    for (int k = 0; k < 9; ++k) tv[k] = t[k];
+    SampleHeader h;
+    FaceVerts f;
+    sample_header(tv, sd, h, f);
+    if (header_too_large(h)) {
+        *count = -1;
+        return;
     }
     int64_t cnt = 0;
     auto emit = [&](const V3& p) {
@@ -2476,37 +2677,34 @@ __global__ void k_sample_triangle(const double* __restrict__ t, double sd, doubl
         }
         ++cnt;
     };
-    double tv[9];
-    for (int k = 0; k < 9; ++k) tv[k] = t[k];
-    SampleHeader h;
-    sample_header(tv, sd, h);
     if (h.trivial) {
-        for (int i = 0; i < 3; ++i) emit(h.vs[i]);
+        for (int i = 0; i < 3; ++i) emit(V3{tv[3 * i], tv[3 * i + 1], tv[3 * i + 2]});
         *count = cnt;
         return;
     }
-    for (int n = 0; n <= h.N; ++n) emit(base_point(h, sd, n));
-    emit(h.v1);
+    for (int n = 0; n <= h.N; ++n) emit(base_point(h, f, sd, n));
+    emit(f.v1);
     if (h.M < 1) {
-        emit(h.v2);
+        emit(f.v2);
         *count = cnt;
         return;
     }
     for (int m = 1; m <= h.M; ++m) {
         V3 v;
         int N1;
-        if (!sample_row(h, sd, m, v, N1)) break;
+        double dd;
+        if (!sample_row(h, f, sd, m, v, N1, dd)) break;
         if (N1 > (int)kMaxSamplesPerRow) {
             *count = -1;
             return;
         }
         for (int i = 0; i <= N1; ++i) emit(row_point(h, v, sd, i));
     }
-    emit(h.v2);
+    emit(f.v2);
     if (h.hasE)
-        for (int n = 1; n <= h.NE; ++n) emit(edge_point(h.v1, h.nE, sd, n));
+        for (int n = 1; n <= h.NE; ++n) emit(edge_point(f.v1, h.n12, sd, n));
     if (h.hasF)
-        for (int n = 1; n <= h.NF; ++n) emit(edge_point(h.v2, h.nF, sd, n));
+        for (int n = 1; n <= h.NF; ++n) emit(edge_point(f.v2, vneg(h.n02), sd, n));
     *count = cnt;
 }
 
