@@ -850,7 +850,7 @@ int tw_newton_stars(tw_ctx* c, const int32_t* star_off, const int32_t* tets, con
     st = sync_status(c, "tw_newton_stars");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "star vertex id out of range");
-    launch_newton_stars_shape(c->newton_shape, c->vx, c->vy, c->vz, doff, dt, dc, nstars,
+    launch_newton_stars_shape(c->newton_shape, c->precision, c->vx, c->vy, c->vz, doff, dt, dc, nstars,
                               c->newton_max_step, c->newton_max_it, dout, dm, c->stream, c->energy_form);
     cudaMemcpyAsync(out, dout, 24 * (size_t)nstars, cudaMemcpyDeviceToHost, c->stream);
     cudaMemcpyAsync(moved, dm, (size_t)nstars, cudaMemcpyDeviceToHost, c->stream);
@@ -923,7 +923,7 @@ int smooth_scratch(tw_ctx* c, int32_t nstars, int64_t ntets, SmoothScratch& S) {
 void smooth_launch(tw_ctx* c, const int32_t* off, const int32_t* tets, const uint8_t* ff,
                    const int32_t* cen, const uint8_t* kinds, int32_t nstars, bool any_surface,
                    double* out, uint8_t* status, const SmoothScratch& S) {
-    launch_smooth_stage1(c->newton_shape, c->vx, c->vy, c->vz, off, tets, cen, kinds, nstars,
+    launch_smooth_stage1(c->newton_shape, c->precision, c->vx, c->vy, c->vz, off, tets, cen, kinds, nstars,
                          c->newton_max_step, c->newton_max_it, out, S.pnew, status, c->stream, c->energy_form);
     if (!any_surface) return;
     cudaMemsetAsync(S.face_count, 0, sizeof(unsigned long long), c->stream);
@@ -1326,7 +1326,7 @@ int tw_newton_stars_device(tw_ctx* c, const int32_t* star_off, const int32_t* te
         return TW_ERR_ARG;
     if (!c->vx) return fail(c, TW_ERR_NO_MESH, "no resident mesh");
     Guard g(c->device);
-    launch_newton_stars_shape(c->newton_shape, c->vx, c->vy, c->vz, star_off, tets, centers,
+    launch_newton_stars_shape(c->newton_shape, c->precision, c->vx, c->vy, c->vz, star_off, tets, centers,
                               nstars, c->newton_max_step, c->newton_max_it, out, moved, c->stream, c->energy_form);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "tw_newton_stars_device");
@@ -1385,7 +1385,7 @@ int tw_newton_autotune_device(tw_ctx* c, const int32_t* star_off, const int32_t*
     if (!c->vx) return fail(c, TW_ERR_NO_MESH, "no resident mesh");
     Guard g(c->device);
     return autotune_shapes(c, "tw_newton_autotune_device", best_shape, ms_per_shape, [&](int sh) {
-        launch_newton_stars_shape(sh, c->vx, c->vy, c->vz, star_off, tets, centers, nstars,
+        launch_newton_stars_shape(sh, c->precision, c->vx, c->vy, c->vz, star_off, tets, centers, nstars,
                                   c->newton_max_step, c->newton_max_it, out, moved, c->stream, c->energy_form);
     });
 }

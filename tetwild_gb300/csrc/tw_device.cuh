@@ -358,6 +358,16 @@ __device__ __forceinline__ double amips_egh_f(const double* T, double* J, double
     return e;
 }
 
+// J and H alone, the operations of amips_egh_f.
+__device__ __forceinline__ void amips_jh_f(const double* T, double* J, double* H, int form) {
+    if (form == TW_ENERGY_FORM_CLOSED) {
+        amips_egh(T, J, H);
+    } else {
+        amips_rf_jacobian(T, J);
+        amips_rf_hessian(T, H);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Exact orientation: CGAL::orientation(p,q,r,s) = sign det[q-p, r-p, s-p].
 // Floating-point filter with Shewchuk's stage-A bound, then exact
@@ -683,6 +693,50 @@ __device__ __forceinline__ Amips32 amips_egh32(const float* d1, const float* d2,
                 }
         }
     }
+    return R;
+}
+
+// Energy alone, with a certified relative bound on its distance from either
+// form's binary64 value: amips_egh32's bound for the exact energy, plus what
+// the binary64 evaluation itself may be off.  M: above every |coordinate|.
+// The reference form works on absolute coordinates: its numerator (12 terms
+// z L with L a difference form) rounds by at most 150 u64 M^2, and its rows b,
+// c by 2^-45 M a component (six roundings of terms up to 1.3 M, and 15-digit
+// coefficients whose sum is off zero by 2e-15 M), so its determinant by
+// 18 2^-45 M times the largest squared component, and 2/3 of that in E; the
+// closed form and the power are far better than the 1e-11 added.
+struct Energy32 {
+    bool ok;
+    float E, rel;   // |E - binary64 E| <= rel * E
+};
+__device__ __forceinline__ Energy32 amips_energy32(const float* d1, const float* d2,
+                                                   const float* d3, float M) {
+    const float isq3 = 0.577350269f, isq6 = 0.408248290f;
+    float a[3], b[3], c[3], A[3], B[3], C[3], NB = 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a[k] = -d3[k];
+        b[k] = fmaf(-2.0f, d1[k], d3[k]) * isq3;
+        c[k] = fmaf(-3.0f, d2[k], d1[k] + d3[k]) * isq6;
+        A[k] = fabsf(d3[k]);
+        B[k] = fmaf(2.0f, fabsf(d1[k]), fabsf(d3[k])) * isq3;
+        C[k] = fmaf(3.0f, fabsf(d2[k]), fabsf(d1[k]) + fabsf(d3[k])) * isq6;
+        NB = fmaf(A[k], A[k], fmaf(B[k], B[k], fmaf(C[k], C[k], NB)));
+    }
+    const float PD = A[0] * fmaf(B[1], C[2], B[2] * C[1]) + A[1] * fmaf(B[2], C[0], B[0] * C[2]) +
+                     A[2] * fmaf(B[0], C[1], B[1] * C[0]);
+    const float N = fmaf(a[2], a[2], fmaf(a[1], a[1], a[0] * a[0])) +
+                    fmaf(b[2], b[2], fmaf(b[1], b[1], b[0] * b[0])) +
+                    fmaf(c[2], c[2], fmaf(c[1], c[1], c[0] * c[0]));
+    const float bc[3] = {fmaf(b[1], c[2], -b[2] * c[1]), fmaf(b[2], c[0], -b[0] * c[2]),
+                         fmaf(b[0], c[1], -b[1] * c[0])};
+    const float D = fmaf(a[2], bc[2], fmaf(a[1], bc[1], a[0] * bc[0]));
+    const float aD = fabsf(D), rN = 1.0f / N, rD = 1.0f / aD;
+    Energy32 R;
+    R.rel = 1.02f * (14.0f * kU32 * NB * rN + 10.6667f * kU32 * PD * rD + 6.0f * kU32 +
+                     1e-13f * M * M * rN + 4e-13f * M * NB * rD + 1e-11f);
+    R.ok = (aD > 1e-18f) && (aD < 1e18f) && (N > 1e-30f) && (N < 1e30f) && (R.rel <= 1e-4f);
+    R.E = R.ok ? N * icbrt32(D * D) : 0.0f;
     return R;
 }
 

@@ -294,16 +294,13 @@ void launch_smooth_project(const Surface& Sin, const Surface& Sb, double eps2,
                            unsigned long long* counters, cudaStream_t s);
 
 // ---- launchers (tw_newton.cu) ----
-void launch_newton_stars(const double* vx, const double* vy, const double* vz,
-                         const int32_t* star_off, const int32_t* tets, const int32_t* centers,
-                         int32_t nstars, int max_step, int max_it, double* out, uint8_t* moved,
-                         cudaStream_t s, int form = TW_ENERGY_FORM_REFERENCE);
-// shape in [0, newton_num_shapes()): lanes per star and block size (see
-// kNewtonShapes); every shape gives bit-identical results.
+// shape in [0, newton_num_shapes()): block size and stars in flight (see
+// kNewtonShapes); precision: the certified mode decides signs and energy
+// comparisons in binary32 where it can.  Every shape and precision gives
+// bit-identical results.
 int newton_num_shapes();
-void newton_shape_info(int shape, int* group, int* block);
-void launch_newton_stars_shape(int shape, const double* vx, const double* vy, const double* vz,
-                               const int32_t* star_off, const int32_t* tets,
+void launch_newton_stars_shape(int shape, int precision, const double* vx, const double* vy,
+                               const double* vz, const int32_t* star_off, const int32_t* tets,
                                const int32_t* centers, int32_t nstars, int max_step, int max_it,
                                double* out, uint8_t* moved, cudaStream_t s,
                                int form = TW_ENERGY_FORM_REFERENCE);
@@ -314,11 +311,11 @@ void launch_newton_stars_shape(int shape, const double* vx, const double* vy, co
 // quality checks at the projected position and the list of one-ring surface
 // faces (appended at face_count; face_base/face_cnt per star); finalize =
 // the face results decide the surface stars.
-void launch_smooth_stage1(int shape, const double* vx, const double* vy, const double* vz,
-                          const int32_t* star_off, const int32_t* tets, const int32_t* centers,
-                          const uint8_t* kinds, int32_t nstars, int max_step, int max_it,
-                          double* out, double* pnew, uint8_t* status, cudaStream_t s,
-                          int form = TW_ENERGY_FORM_REFERENCE);
+void launch_smooth_stage1(int shape, int precision, const double* vx, const double* vy,
+                          const double* vz, const int32_t* star_off, const int32_t* tets,
+                          const int32_t* centers, const uint8_t* kinds, int32_t nstars,
+                          int max_step, int max_it, double* out, double* pnew, uint8_t* status,
+                          cudaStream_t s, int form = TW_ENERGY_FORM_REFERENCE);
 void launch_smooth_stage2(int shape, const double* vx, const double* vy, const double* vz,
                           const int32_t* star_off, const int32_t* tets, const uint8_t* face_flags,
                           const int32_t* centers, int32_t nstars, const double* pnew,

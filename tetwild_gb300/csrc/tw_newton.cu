@@ -10,145 +10,15 @@
 // The 3x3 solve is Householder QR with column pivoting (Golub & Van Loan,
 // Alg. 5.4.1), the same operations as the oracle's, standing in for Eigen's
 // ColPivHouseholderQR (:492).
+#include <algorithm>
+
 #include "tw_device.cuh"
 #include "tw_internal.h"
 #include "tw_star.cuh"
 
 namespace tw {
 
-__global__ void __launch_bounds__(128) k_newton_stars(const double* __restrict__ vx,
-                                                      const double* __restrict__ vy,
-                                                      const double* __restrict__ vz,
-                                                      const int32_t* __restrict__ star_off,
-                                                      const int4* __restrict__ tets,
-                                                      const int32_t* __restrict__ centers,
-                                                      int32_t nstars, int max_step, int max_it,
-                                                      double* __restrict__ out,
-                                                      uint8_t* __restrict__ moved, int form) {
-    int32_t sid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (sid >= nstars) return;
-    int32_t b = star_off[sid], e = star_off[sid + 1];
-    StarView S{vx, vy, vz, tets + b, e - b, centers[sid], form};
-    double pos[3] = {vx[S.v], vy[S.v], vz[S.v]};
-    int is_moved = 0;
-    double old_energy = 0.0, new_energy = 0.0, J[3], H[9];
-    for (int step = 0; step < max_step; ++step) {
-        if (!star_update(S, pos, old_energy, J, H)) break;
-        double old_pf[3] = {pos[0], pos[1], pos[2]};
-        double X0[3] = {pos[0], pos[1], pos[2]};
-        double a = 1.0;
-        bool step_taken = false;
-        for (int it = 0; it < max_it; ++it) {
-            double rhs[3], X[3];
-            for (int i = 0; i < 3; ++i)
-                rhs[i] = ((H[3 * i] * X0[0] + H[3 * i + 1] * X0[1]) + H[3 * i + 2] * X0[2]) - a * J[i];
-            qr_solve3(H, rhs, X);
-            if (!isfinite(X[0]) || !isfinite(X[1]) || !isfinite(X[2])) {
-                a /= 2.0;
-                continue;
-            }
-            pos[0] = X[0];
-            pos[1] = X[1];
-            pos[2] = X[2];
-            if (star_flip(S, pos)) {
-                pos[0] = old_pf[0];
-                pos[1] = old_pf[1];
-                pos[2] = old_pf[2];
-                a /= 2.0;
-                continue;
-            }
-            new_energy = star_new_energy(S, pos);
-            if (new_energy >= old_energy || isinf(new_energy) || isnan(new_energy)) {
-                pos[0] = old_pf[0];
-                pos[1] = old_pf[1];
-                pos[2] = old_pf[2];
-                a /= 2.0;
-                continue;
-            }
-            step_taken = true;
-            break;
-        }
-        if (fabs(new_energy - old_energy) < 1e-5) step_taken = false;
-        if (!step_taken) {
-            is_moved = (step != 0);
-            break;
-        }
-        is_moved = 1;
-    }
-    out[3 * (int64_t)sid] = pos[0];
-    out[3 * (int64_t)sid + 1] = pos[1];
-    out[3 * (int64_t)sid + 2] = pos[2];
-    moved[sid] = (uint8_t)is_moved;
-}
-
-template <int G>
-__global__ void __launch_bounds__(256) k_newton_group(const double* __restrict__ vx,
-                                                      const double* __restrict__ vy,
-                                                      const double* __restrict__ vz,
-                                                      const int32_t* __restrict__ star_off,
-                                                      const int4* __restrict__ tets,
-                                                      const int32_t* __restrict__ centers,
-                                                      int32_t nstars, int max_step, int max_it,
-                                                      double* __restrict__ out,
-                                                      uint8_t* __restrict__ moved, int form) {
-    const int lane = threadIdx.x & 31;
-    const int gl = lane & (G - 1);
-    const unsigned gm = group_mask<G>(lane);
-    const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const int64_t ngroups = ((int64_t)gridDim.x * blockDim.x) / G;
-    for (int64_t sid = gid; sid < nstars; sid += ngroups) {
-        const int32_t b = star_off[sid], nt = star_off[sid + 1] - b;
-        StarView S{vx, vy, vz, tets + b, nt, centers[sid], form};
-        double pos[3] = {vx[S.v], vy[S.v], vz[S.v]};
-        const int is_moved = newton_group_star<G>(S, pos, max_step, max_it, gl, gm);
-        if (gl == 0) {
-            out[3 * sid] = pos[0];
-            out[3 * sid + 1] = pos[1];
-            out[3 * sid + 2] = pos[2];
-            moved[sid] = (uint8_t)is_moved;
-        }
-    }
-}
-
-template <int G>
-__global__ void __launch_bounds__(256) k_smooth_stage1(
-    const double* __restrict__ vx, const double* __restrict__ vy, const double* __restrict__ vz,
-    const int32_t* __restrict__ star_off, const int4* __restrict__ tets,
-    const int32_t* __restrict__ centers, const uint8_t* __restrict__ kinds, int32_t nstars,
-    int max_step, int max_it, double* __restrict__ out, double* __restrict__ pnew,
-    uint8_t* __restrict__ status, int form) {
-    const int lane = threadIdx.x & 31;
-    const int gl = lane & (G - 1);
-    const unsigned gm = group_mask<G>(lane);
-    const int64_t gid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G;
-    const int64_t ngroups = ((int64_t)gridDim.x * blockDim.x) / G;
-    for (int64_t sid = gid; sid < nstars; sid += ngroups) {
-        const int32_t b = star_off[sid], nt = star_off[sid + 1] - b;
-        StarView S{vx, vy, vz, tets + b, nt, centers[sid], form};
-        const double p0[3] = {vx[S.v], vy[S.v], vz[S.v]};
-        double pos[3] = {p0[0], p0[1], p0[2]};
-        const uint8_t kind = kinds ? kinds[sid] : (uint8_t)TW_STAR_INTERIOR;
-        const bool surface = (kind == TW_STAR_SURFACE || kind == TW_STAR_BOUNDARY);
-        uint8_t st;
-        if (!star_positive<G>(S, p0, gl, gm)) {
-            st = TW_SMOOTH_INVALID;
-        } else if (!newton_group_star<G>(S, pos, max_step, max_it, gl, gm)) {
-            st = TW_SMOOTH_NOT_MOVED;
-        } else {
-            st = surface ? kSmoothPendingProject : (uint8_t)TW_SMOOTH_MOVED;
-        }
-        if (gl == 0) {
-            const bool moved = (st == TW_SMOOTH_MOVED);
-            out[3 * sid] = moved ? pos[0] : p0[0];
-            out[3 * sid + 1] = moved ? pos[1] : p0[1];
-            out[3 * sid + 2] = moved ? pos[2] : p0[2];
-            pnew[3 * sid] = pos[0];
-            pnew[3 * sid + 1] = pos[1];
-            pnew[3 * sid + 2] = pos[2];
-            status[sid] = st;
-        }
-    }
-}
+#include "tw_wave.cuh"
 
 template <int G>
 __global__ void __launch_bounds__(256) k_smooth_stage2(
@@ -430,78 +300,58 @@ __global__ void k_smooth_finalize(int32_t nstars, const int32_t* __restrict__ fa
     }
 }
 
-// Launch shape of the fused step: lanes per star (8, 16, 32) and threads per
-// block (64, 128, 256); variant 0 is the one-thread-per-star kernel.
+// Launch shapes: threads per block of the Newton kernel (64, 128, 256) and
+// lanes per star (8, 16, 32) of the smoothing and collapse stages; the Newton
+// kernel keeps 4 block / lanes stars a block in flight, at most 32 (shape 0,
+// once a thread per star, equals shape 2).
 struct NewtonShape {
     int group;
     int block;
 };
-static const NewtonShape kNewtonShapes[] = {{1, 128},  {8, 64},   {8, 128},  {8, 256},
+static const NewtonShape kNewtonShapes[] = {{8, 128},  {8, 64},   {8, 128},  {8, 256},
                                             {16, 64},  {16, 128}, {16, 256}, {32, 64},
                                             {32, 128}, {32, 256}};
 int newton_num_shapes() { return (int)(sizeof(kNewtonShapes) / sizeof(kNewtonShapes[0])); }
-void newton_shape_info(int shape, int* group, int* block) {
+
+static int smooth_group(int shape, int* block) {
     if (shape < 0 || shape >= newton_num_shapes()) shape = 5;
-    *group = kNewtonShapes[shape].group;
     *block = kNewtonShapes[shape].block;
+    return kNewtonShapes[shape].group;
 }
 
-void launch_newton_stars_shape(int shape, const double* vx, const double* vy, const double* vz,
-                               const int32_t* star_off, const int32_t* tets,
+template <bool SMOOTH, bool CERT>
+static void launch_wave(int shape, WaveArgs A, cudaStream_t s) {
+    int block;
+    const int group = smooth_group(shape, &block);
+    A.slots = std::min(kWaveSlots, 4 * block / group);
+    // one star a block before two: the grid fills the SMs first
+    const int grid = grid_for(A.nstars, 1, 512 / block);
+    if (block == 64) k_newton_wave<SMOOTH, CERT, 64><<<grid, 64, 0, s>>>(A);
+    else if (block == 128) k_newton_wave<SMOOTH, CERT, 128><<<grid, 128, 0, s>>>(A);
+    else k_newton_wave<SMOOTH, CERT, 256><<<grid, 256, 0, s>>>(A);
+}
+
+void launch_newton_stars_shape(int shape, int precision, const double* vx, const double* vy,
+                               const double* vz, const int32_t* star_off, const int32_t* tets,
                                const int32_t* centers, int32_t nstars, int max_step, int max_it,
                                double* out, uint8_t* moved, cudaStream_t s, int form) {
     if (nstars <= 0) return;
-    if (shape < 0 || shape >= newton_num_shapes()) shape = 5;
-    const NewtonShape sh = kNewtonShapes[shape];
-    const int4* t4 = reinterpret_cast<const int4*>(tets);
-    if (sh.group == 1) {
-        int grid = (nstars + sh.block - 1) / sh.block;
-        k_newton_stars<<<grid, sh.block, 0, s>>>(vx, vy, vz, star_off, t4, centers, nstars,
-                                                 max_step, max_it, out, moved, form);
-        return;
-    }
-    const int64_t threads = (int64_t)nstars * sh.group;
-    const int grid = grid_for(threads, sh.block, 2048 / sh.block);
-    if (sh.group == 8)
-        k_newton_group<8><<<grid, sh.block, 0, s>>>(vx, vy, vz, star_off, t4, centers, nstars,
-                                                    max_step, max_it, out, moved, form);
-    else if (sh.group == 16)
-        k_newton_group<16><<<grid, sh.block, 0, s>>>(vx, vy, vz, star_off, t4, centers, nstars,
-                                                     max_step, max_it, out, moved, form);
-    else
-        k_newton_group<32><<<grid, sh.block, 0, s>>>(vx, vy, vz, star_off, t4, centers, nstars,
-                                                     max_step, max_it, out, moved, form);
+    const WaveArgs A{vx, vy, vz, star_off, reinterpret_cast<const int4*>(tets), centers, nullptr,
+                     nstars, max_step, max_it, 0, form, out, nullptr, moved};
+    if (precision == TW_PRECISION_FP32_CERTIFIED) launch_wave<false, true>(shape, A, s);
+    else launch_wave<false, false>(shape, A, s);
 }
 
-// Smoothing kernels use the Newton shape's group size; shape 0 (one thread
-// per star) runs them with 8 lanes.
-static int smooth_group(int shape, int* block) {
-    if (shape < 0 || shape >= newton_num_shapes()) shape = 5;
-    NewtonShape sh = kNewtonShapes[shape];
-    if (sh.group == 1) sh = NewtonShape{8, 128};
-    *block = sh.block;
-    return sh.group;
-}
-
-void launch_smooth_stage1(int shape, const double* vx, const double* vy, const double* vz,
-                          const int32_t* star_off, const int32_t* tets, const int32_t* centers,
-                          const uint8_t* kinds, int32_t nstars, int max_step, int max_it,
-                          double* out, double* pnew, uint8_t* status, cudaStream_t s,
-                          int form) {
+void launch_smooth_stage1(int shape, int precision, const double* vx, const double* vy,
+                          const double* vz, const int32_t* star_off, const int32_t* tets,
+                          const int32_t* centers, const uint8_t* kinds, int32_t nstars,
+                          int max_step, int max_it, double* out, double* pnew, uint8_t* status,
+                          cudaStream_t s, int form) {
     if (nstars <= 0) return;
-    int block;
-    const int G = smooth_group(shape, &block);
-    const int grid = grid_for((int64_t)nstars * G, block, 2048 / block);
-    const int4* t4 = reinterpret_cast<const int4*>(tets);
-    if (G == 8)
-        k_smooth_stage1<8><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, centers, kinds, nstars,
-                                                  max_step, max_it, out, pnew, status, form);
-    else if (G == 16)
-        k_smooth_stage1<16><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, centers, kinds, nstars,
-                                                   max_step, max_it, out, pnew, status, form);
-    else
-        k_smooth_stage1<32><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, centers, kinds, nstars,
-                                                   max_step, max_it, out, pnew, status, form);
+    const WaveArgs A{vx, vy, vz, star_off, reinterpret_cast<const int4*>(tets), centers, kinds,
+                     nstars, max_step, max_it, 0, form, out, pnew, status};
+    if (precision == TW_PRECISION_FP32_CERTIFIED) launch_wave<true, true>(shape, A, s);
+    else launch_wave<true, false>(shape, A, s);
 }
 
 void launch_smooth_stage2(int shape, const double* vx, const double* vy, const double* vz,
@@ -567,14 +417,6 @@ void launch_collapse_finalize(int32_t n, const int32_t* face_base, const int32_t
     if (n <= 0) return;
     k_collapse_finalize<<<grid_for(n, 256, 8), 256, 0, s>>>(n, face_base, face_cnt, face_out,
                                                             status);
-}
-
-void launch_newton_stars(const double* vx, const double* vy, const double* vz,
-                         const int32_t* star_off, const int32_t* tets, const int32_t* centers,
-                         int32_t nstars, int max_step, int max_it, double* out, uint8_t* moved,
-                         cudaStream_t s, int form) {
-    launch_newton_stars_shape(5, vx, vy, vz, star_off, tets, centers, nstars, max_step, max_it, out,
-                              moved, s, form);
 }
 
 }  // namespace tw

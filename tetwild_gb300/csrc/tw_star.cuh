@@ -1,7 +1,7 @@
 // tw_star.cuh -- device routines of one-ring stars used by the Newton,
 // smoothing and collapse kernels (tw_newton.cu):
-// the 3x3 solve, the star view and gathers, NewtonsMethod for G lanes, the
-// inversion and quality checks and the one-ring surface faces.
+// the 3x3 solve, the star view and gathers, the inversion and quality checks
+// and the one-ring surface faces.
 #pragma once
 
 #include "tw_device.cuh"
@@ -110,170 +110,14 @@ __device__ __forceinline__ void gather_tet(const StarView& S, int4 tv, int start
     }
 }
 
-static __device__ bool star_flip(const StarView& S, const double* pos) {
-    double T[12];
-    for (int32_t i = 0; i < S.nt; ++i) {
-        gather_tet(S, __ldg(S.tets + i), 0, pos, T);
-        if (orient3d(T, T + 3, T + 6, T + 9) != 1) return true;
-    }
-    return false;
+// Position of vertex v in the tet (0 when it is none of the four).
+__device__ __forceinline__ int centre_index(int4 tv, int32_t v) {
+    return (tv.x == v) ? 0 : (tv.y == v) ? 1 : (tv.z == v) ? 2 : (tv.w == v) ? 3 : 0;
 }
 
-static __device__ double star_new_energy(const StarView& S, const double* pos) {
-    double s = 0.0, T[12];
-    for (int32_t i = 0; i < S.nt; ++i) {
-        gather_tet(S, __ldg(S.tets + i), 0, pos, T);
-        s += amips_energy_f(T, S.form);
-    }
-    if (isinf(s) || isnan(s) || s <= 0.0 || s > kMaxEnergy) s = kMaxEnergy;
-    return s;
-}
-
-static __device__ bool star_update(const StarView& S, const double* pos, double& energy, double* J,
-                            double* H) {
-    double e = 0.0, T[12], J1[3], H1[9];
-    for (int k = 0; k < 3; ++k) J[k] = 0.0;
-    for (int k = 0; k < 9; ++k) H[k] = 0.0;
-    for (int32_t i = 0; i < S.nt; ++i) {
-        int4 tv = __ldg(S.tets + i);
-        int start = (tv.x == S.v) ? 0 : (tv.y == S.v) ? 1 : (tv.z == S.v) ? 2 : (tv.w == S.v) ? 3 : 0;
-        gather_tet(S, tv, start, pos, T);
-        e += amips_egh_f(T, J1, H1, S.form);   // its E is amips_energy_f's, operation for operation
-        for (int j = 0; j < 3; ++j) {
-            J[j] += J1[j];
-            H[3 * j + 0] += H1[3 * j + 0];
-            H[3 * j + 1] += H1[3 * j + 1];
-            H[3 * j + 2] += H1[3 * j + 2];
-        }
-    }
-    if (isinf(e)) e = kMaxEnergy;
-    energy = e;
-    if (isnan(e)) return false;
-    if (e <= 0.0) return false;
-    for (int k = 0; k < 3; ++k)
-        if (!isfinite(J[k])) return false;
-    for (int k = 0; k < 9; ++k)
-        if (!isfinite(H[k])) return false;
-    return true;
-}
-
-// ---------------------------------------------------------------------------
-// Fused Newton step with G lanes per star (G = 8, 16 or 32).
-//
-// The lanes of a group evaluate the star's tets G at a time; the per-tet
-// terms are then added in tet order by broadcasting lane 0's value first,
-// lane 1's next, ...: every lane accumulates the same sequence, so every lane
-// holds the sum rounded exactly as the sequential loops of the reference
-// (VertexSmoother.cpp:654-672 for E/J/H, :606-614 for the trial energy).
-// The QR solve, the step logic and the acceptance tests are evaluated
-// redundantly by all lanes of the group (uniform within the group); a trial
-// position is rejected if any lane finds an inverted tet.
-// ---------------------------------------------------------------------------
 template <int G>
 __device__ __forceinline__ unsigned group_mask(int lane) {
     return (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-}
-
-// NewtonsMethod for the star S with G lanes; every lane returns the same
-// position and is_moved.
-template <int G>
-__device__ __forceinline__ int newton_group_star(const StarView& S, double* pos, int max_step,
-                                                 int max_it, int gl, unsigned gm) {
-    const int32_t nt = S.nt;
-    int is_moved = 0;
-    double old_energy = 0.0, new_energy = 0.0, J[3], H[9];
-    for (int step = 0; step < max_step; ++step) {
-        // NewtonsUpdate: E, J, H summed over the tets in caller order
-        double e = 0.0;
-        for (int k = 0; k < 3; ++k) J[k] = 0.0;
-        for (int k = 0; k < 9; ++k) H[k] = 0.0;
-        for (int c0 = 0; c0 < nt; c0 += G) {
-            const int cnt = min(G, nt - c0);
-            double te = 0.0, tJ[3] = {0.0, 0.0, 0.0}, tH[9];
-            for (int k = 0; k < 9; ++k) tH[k] = 0.0;
-            if (gl < cnt) {
-                int4 tv = __ldg(S.tets + c0 + gl);
-                int start = (tv.x == S.v) ? 0 : (tv.y == S.v) ? 1 : (tv.z == S.v) ? 2
-                          : (tv.w == S.v) ? 3 : 0;
-                double T[12];
-                gather_tet(S, tv, start, pos, T);
-                te = amips_egh_f(T, tJ, tH, S.form);   // its E is amips_energy_f's
-            }
-            for (int t = 0; t < cnt; ++t) {
-                e += __shfl_sync(gm, te, t, G);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) J[k] += __shfl_sync(gm, tJ[k], t, G);
-#pragma unroll
-                for (int k = 0; k < 9; ++k) H[k] += __shfl_sync(gm, tH[k], t, G);
-            }
-        }
-        if (isinf(e)) e = kMaxEnergy;
-        old_energy = e;
-        bool ok = !isnan(e) && !(e <= 0.0);
-        for (int k = 0; k < 3; ++k) ok = ok && isfinite(J[k]);
-        for (int k = 0; k < 9; ++k) ok = ok && isfinite(H[k]);
-        if (!ok) break;
-        double old_pf[3] = {pos[0], pos[1], pos[2]};
-        double X0[3] = {pos[0], pos[1], pos[2]};
-        double a = 1.0;
-        bool step_taken = false;
-        for (int it = 0; it < max_it; ++it) {
-            double rhs[3], X[3];
-            for (int i = 0; i < 3; ++i)
-                rhs[i] = ((H[3 * i] * X0[0] + H[3 * i + 1] * X0[1]) + H[3 * i + 2] * X0[2]) -
-                         a * J[i];
-            qr_solve3(H, rhs, X);
-            if (!isfinite(X[0]) || !isfinite(X[1]) || !isfinite(X[2])) {
-                a /= 2.0;
-                continue;
-            }
-            pos[0] = X[0];
-            pos[1] = X[1];
-            pos[2] = X[2];
-            bool flip = false;
-            for (int c0 = gl; c0 < nt; c0 += G) {
-                double T[12];
-                gather_tet(S, __ldg(S.tets + c0), 0, pos, T);
-                flip = flip || (orient3d(T, T + 3, T + 6, T + 9) != 1);
-            }
-            if (__any_sync(gm, flip)) {
-                pos[0] = old_pf[0];
-                pos[1] = old_pf[1];
-                pos[2] = old_pf[2];
-                a /= 2.0;
-                continue;
-            }
-            double sum = 0.0;
-            for (int c0 = 0; c0 < nt; c0 += G) {
-                const int cnt = min(G, nt - c0);
-                double te = 0.0;
-                if (gl < cnt) {
-                    double T[12];
-                    gather_tet(S, __ldg(S.tets + c0 + gl), 0, pos, T);
-                    te = amips_energy_f(T, S.form);
-                }
-                for (int t = 0; t < cnt; ++t) sum += __shfl_sync(gm, te, t, G);
-            }
-            if (isinf(sum) || isnan(sum) || sum <= 0.0 || sum > kMaxEnergy) sum = kMaxEnergy;
-            new_energy = sum;
-            if (new_energy >= old_energy || isinf(new_energy) || isnan(new_energy)) {
-                pos[0] = old_pf[0];
-                pos[1] = old_pf[1];
-                pos[2] = old_pf[2];
-                a /= 2.0;
-                continue;
-            }
-            step_taken = true;
-            break;
-        }
-        if (fabs(new_energy - old_energy) < 1e-5) step_taken = false;
-        if (!step_taken) {
-            is_moved = (step != 0);
-            break;
-        }
-        is_moved = 1;
-    }
-    return is_moved;
 }
 
 // ---------------------------------------------------------------------------
