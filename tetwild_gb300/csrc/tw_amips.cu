@@ -173,12 +173,12 @@ __global__ void __launch_bounds__(128) k_amips_recheck(
         } else if (part == 1) {
             if (J) {
                 double jv[3];
-                amips_rf_jacobian(t, jv);
+                amips_rf<false>(t, jv, nullptr);
                 for (int c = 0; c < 3; ++c) J[(int64_t)c * n + i] = jv[c];
             }
         } else if (H) {
             double hv[9];
-            amips_rf_hessian(t, hv);
+            amips_rf<false>(t, nullptr, hv);
             for (int c = 0; c < 9; ++c) H[(int64_t)c * n + i] = hv[c];
         }
     }

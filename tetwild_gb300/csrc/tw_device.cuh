@@ -18,7 +18,73 @@ constexpr double kIsq6 = 0.40824829046386301637;       // 1/sqrt(6)
 constexpr double kTwoThirds = 0.66666666666666662966;
 constexpr double kTenNinths = 1.1111111111111111605;
 constexpr double kEps = 1.1102230246251565404e-16;     // 2^-53
+constexpr float kU32 = 5.9604644775390625e-08f;  // 2^-24
 constexpr double kO3dBound = (7.0 + 56.0 * kEps) * kEps;  // Shewchuk 1997, orient3d stage A
+
+// ---------------------------------------------------------------------------
+// binary32 <-> binary64 conversions in integer arithmetic.  On this GPU the
+// hardware conversions issue to the (slow) FP64 pipe; these use only the
+// integer ALU, for every class of input (normal, subnormal, zero, infinity,
+// NaN), and agree with the hardware bit for bit (tw_self_test checks it).
+// ---------------------------------------------------------------------------
+// Exact: every binary32 value is a binary64 value.
+__device__ __forceinline__ double f2d_exact(float f) {
+    uint32_t b = __float_as_uint(f);
+    uint32_t s = b & 0x80000000u;
+    uint32_t e = (b >> 23) & 0xffu;
+    uint32_t m = b & 0x7fffffu;
+    uint32_t hi, lo;
+    if (e == 0xffu) {            // inf / NaN: payload kept
+        hi = s | 0x7ff00000u | (m >> 3);
+        lo = m << 29;
+    } else if (e != 0u) {        // normal
+        hi = s | ((e + (1023u - 127u)) << 20) | (m >> 3);
+        lo = m << 29;
+    } else if (m == 0u) {        // signed zero
+        hi = s;
+        lo = 0u;
+    } else {                     // subnormal: m * 2^-149, top bit at position p
+        uint32_t p = 31u - (uint32_t)__clz(m);
+        unsigned long long mant = ((unsigned long long)m << (52u - p)) & 0x000fffffffffffffULL;
+        hi = s | ((p + 1023u - 149u) << 20) | (uint32_t)(mant >> 32);
+        lo = (uint32_t)mant;
+    }
+    return __hiloint2double((int)hi, (int)lo);
+}
+// Round to nearest, ties to even (the IEEE default), like __double2float_rn.
+__device__ __forceinline__ float d2f_rn(double x) {
+    unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
+    uint32_t s = hi & 0x80000000u;
+    uint32_t e11 = (hi >> 20) & 0x7ffu;
+    if (e11 == 0x7ffu) {                               // inf / NaN (NaN made quiet)
+        bool nan = ((hi & 0xfffffu) | lo) != 0u;
+        return __uint_as_float(s | 0x7f800000u | (nan ? 0x00400000u | ((hi & 0xfffffu) << 3) | (lo >> 29) : 0u));
+    }
+    int e = (int)e11 - 1023 + 127;
+    if (e >= 255) return __uint_as_float(s | 0x7f800000u);   // overflow: inf
+    if (e >= 1) {                                       // normal result
+        uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29);  // top 23 mantissa bits
+        uint32_t rest = lo & 0x1fffffffu;                  // the 29 dropped bits
+        uint32_t r = ((uint32_t)e << 23) | m;
+        // a carry out of the mantissa increments the exponent (and rounds to
+        // inf at the top of the range), as round-to-nearest requires
+        r += (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
+        return __uint_as_float(s | r);
+    }
+    // subnormal or zero result: value = M53 * 2^(e11 - 1075) = k * 2^-149
+    if (e11 == 0u) return __uint_as_float(s);          // double zero or subnormal
+    unsigned long long M = (b & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
+    uint32_t sh = 926u - e11;                           // >= 30 here
+    if (sh > 54u) return __uint_as_float(s);            // below half the smallest subnormal
+    unsigned long long k = M >> sh;
+    unsigned long long rest = M & ((1ULL << sh) - 1ULL);
+    unsigned long long half = 1ULL << (sh - 1u);
+    k += (rest > half || (rest == half && (k & 1ULL))) ? 1ULL : 0ULL;
+    return __uint_as_float(s | (uint32_t)k);            // k = 2^23 is the smallest normal
+}
+
+#include "tw_exact.cuh"
 
 // ---------------------------------------------------------------------------
 // x^(-1/3) for x >= 0: exponent reduction to m in [1,8), three binary32 and
@@ -187,7 +253,7 @@ constexpr double kRfLn2 = 0.6931471805599453;
 // s^(-0.333333333333333): s^(-1/3) (icbrt) times the first-order factor
 // 1 + kRfDelta ln s (a correction below 2.6e-13 over the double range; ln s
 // to ~4% from the exponent and one atanh term keeps its error below 1e-17).
-__device__ __forceinline__ double rf_pow_m13(double s) {
+static __device__ __noinline__ double rf_pow_m13_plain(double s) {
     const double r = icbrt(s);
     if (!(r > 0.0) || isinf(r)) return r;
     const unsigned long long u = (unsigned long long)__double_as_longlong(s);
@@ -198,7 +264,75 @@ __device__ __forceinline__ double rf_pow_m13(double s) {
     return r + r * (kRfDelta * ln);
 }
 
-__device__ __forceinline__ double amips_rf_energy(const double* T) {
+// The same value (every operation's rounding included) in 10 binary64
+// instructions instead of 37: the conversions and the scaling by a power of
+// two are integer operations, and the last Newton correction and the
+// correction by kRfDelta ln s (up to some hundred units of the last place)
+// are rounded as in tw_exact.cuh.
+__device__ __forceinline__ double rf_pow_m13(double s) {
+    const uint32_t hi = (uint32_t)__double2hiint(s), lo = (uint32_t)__double2loint(s);
+    if (hi - 0x00100000u >= 0x7fe00000u) return rf_pow_m13_plain(s);   // not a positive normal
+    const int ex = (int)(hi >> 20) - 1023;
+    const int q = (int)((uint32_t)(ex + 3072) / 3u) - 1024, rem = ex - 3 * q;   // floor(ex / 3)
+    const double m = __hiloint2double((int)((hi & 0xfffffu) | (uint32_t)(1023 + rem) << 20), (int)lo);
+    uint32_t mb = ((uint32_t)(127 + rem) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+    const uint32_t rest = lo & 0x1fffffffu;
+    mb += (rest > 0x10000000u || (rest == 0x10000000u && (mb & 1u))) ? 1u : 0u;
+    const float mf = __uint_as_float(mb);   // m to nearest
+    float yf = 0.9318f - 0.06015f * mf;
+    const float third_f = 0.333333343f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float y3 = (yf * yf) * yf;
+        const float t = 1.0f - mf * y3;
+        yf = yf + (yf * t) * third_f;
+    }
+    const uint32_t yb = __float_as_uint(yf);
+    double y = __hiloint2double((int)((((yb >> 23) + 896u) << 20) | ((yb & 0x7fffffu) >> 3)),
+                                (int)(yb << 29));
+    {
+        const double y3 = (y * y) * y;
+        const double t = 1.0 - m * y3;
+        y = y + (y * t) * 0.33333333333333331483;
+    }
+    const double p = m * ((y * y) * y);
+    // t = 1 - p is exact: a whole number of 2^-53 below 1, of 2^-52 above
+    const long long d = 0x3ff0000000000000LL - __double_as_longlong(p);
+    bool ok = d > -(1LL << 23) && d < (1LL << 23) && exponent_field(y) == 1022;
+    // y t / 3 in units 2^-53 of y = (ys + yl) / 2, to 2^-44: the seed's error leaves
+    // up to some million units for m near 1 or 8
+    const float ys = significand32(y), yl = (float)(__double2loint(y) & 0x1fffffff) * 0x1p-52f;
+    const float df = 0.5f * (float)(int)(d >= 0 ? d : d + d);
+    const float ph = df * ys, pl = fmaf(df, yl, fmaf(df, ys, -ph));
+    const float g1 = ph * third_f;
+    const float gl = fmaf(ph, third_f, -g1) + fmaf(ph, -9.93410747e-9f, pl * third_f);
+    y = add_units(y, g1, gl, fmaf(fabsf(g1), 1e-9f, 1e-6f), ok);
+    const double r = __hiloint2double(__double2hiint(y) - q * 0x100000, __double2loint(y));
+    // r kRfDelta ln s in units of r: 2^52 kRfDelta = 1.58333
+    const float ms = significand32(s);
+    const float ln = fmaf((float)ex, 0.693147181f, __fdividef(2.0f * (ms - 1.0f), ms + 1.0f));
+    const float g2 = ys * (1.58333333f * ln);
+    const double out = add_units(r, g2, 0.0f, fmaf(fabsf((float)ex), 1e-6f, 4e-6f), ok);
+    return ok ? out : rf_pow_m13_plain(s);
+}
+
+// The forms L of the numerator are evaluated doubled, x1 + x2 + x3 - 3 x0 for
+// 0.5 x1 + 0.5 x2 - 1.5 x0 + 0.5 x3 and so on: scaling every operand by two
+// scales every rounded result by two, and 3 x0 serves the gradient too.  That
+// holds away from overflow and underflow: coordinates whose largest magnitude
+// lies outside 2^-400 .. 2^400 take the expressions as the reference has them
+// (amips_rf_*_plain).  E, J, H and the sign of a tet took 673 binary64 warp
+// instructions, now 555: 1M tets in 1.10 ms instead of 1.31 (the binary64 pipe
+// 84% busy in both).
+__device__ __forceinline__ int coord_exponent(const double* T) {
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) m = max(m, __double2hiint(T[k]) & 0x7fffffff);
+    return m >> 20;   // field of the largest magnitude
+}
+__device__ __forceinline__ bool coords_in_range(int e) { return e > 623 && e < 1423; }
+
+static __device__ __noinline__ double amips_rf_energy_plain(const double* T) {
     const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
     const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
     const double bx = (kRfB1 * x0 - kRfB2 * x1) + kRfB1 * x3;
@@ -219,10 +353,10 @@ __device__ __forceinline__ double amips_rf_energy(const double* T) {
         y2 * (((0.5 * y3 + 0.5 * y0) + 0.5 * y1) - 1.5 * y2);
     const double det = ((z0 - z3) * (cy * bx - by * cx) - (y0 - y3) * (cz * bx - cx * bz)) +
                        (x0 - x3) * (by * cz - cy * bz);
-    return -num * rf_pow_m13((det * det));
+    return -num * rf_pow_m13_plain((det * det));
 }
 
-__device__ __forceinline__ void amips_rf_jacobian(const double* T, double* J) {
+static __device__ __noinline__ void amips_rf_jacobian_plain(const double* T, double* J) {
     const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
     const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
     const double dy = y0 - y3, dz = z0 - z3, dx = x0 - x3;
@@ -235,7 +369,7 @@ __device__ __forceinline__ void amips_rf_jacobian(const double* T, double* J) {
     const double czbx = cz * bx - bz * cx;
     const double cybx = cy * bx, cxby = cx * by;
     const double det = (czbx * dy - dz * (cybx - cxby)) - dx * (cz * by - bz * cy);
-    const double r = rf_pow_m13((det * det));
+    const double r = rf_pow_m13_plain((det * det));
     const double sz = kRfS2 * z1 - kRfS2 * z2, sy = kRfS2 * y1 - kRfS2 * y2;
     const double sx = kRfS2 * x1 - kRfS2 * x2;
     const double hx = 0.5 * x2 + 0.5 * x1, hy = 0.5 * y1 + 0.5 * y2, hz = 0.5 * z1 + 0.5 * z2;
@@ -254,7 +388,7 @@ __device__ __forceinline__ void amips_rf_jacobian(const double* T, double* J) {
     J[2] = r * (((((-z1) - z2) - z3) + w * (((-(dy * sx)) - cybx) + cxby + dx * sy)) + 3.0 * z0);
 }
 
-__device__ __forceinline__ void amips_rf_hessian(const double* T, double* H) {
+static __device__ __noinline__ void amips_rf_hessian_plain(const double* T, double* H) {
     const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
     const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
     const double dz = z0 - z3, dx = x0 - x3, dy = y0 - y3;
@@ -274,7 +408,7 @@ __device__ __forceinline__ void amips_rf_hessian(const double* T, double* H) {
     const double mz = dy * mxz;
     const double det = (mx + my) - mz;
     const double det2 = (det * det);
-    const double r = rf_pow_m13(det2);
+    const double r = rf_pow_m13_plain(det2);
     const double lx = ((x2 - 3.0 * x0) + x1) + x3;
     const double sy = kRfS2 * y1 - kRfS2 * y2;
     const double dzsy = dz * sy;
@@ -342,6 +476,220 @@ __device__ __forceinline__ void amips_rf_hessian(const double* T, double* H) {
     H[8] = r * ((((-lz) * t) * k43 - (kRf10_9 * (t * t)) * nd) + 3.0);
 }
 
+// The same values, operation for operation, in fewer binary64 instructions, for
+// coordinates in range (ce: coord_exponent(T)).
+__device__ __forceinline__ double amips_rf_energy_in(const double* T) {
+    const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
+    const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
+    const double bx = (kRfB1 * x0 - kRfB2 * x1) + kRfB1 * x3;
+    const double cy = ((kRfC1 * y3 + kRfC1 * y0) + kRfC1 * y1) - kRfC3 * y2;
+    const double by = (kRfB1 * y3 + kRfB1 * y0) - kRfB2 * y1;
+    const double cx = ((kRfC1 * x0 - kRfC3 * x2) + kRfC1 * x1) + kRfC1 * x3;
+    const double cz = ((kRfC1 * z0 + kRfC1 * z1) - kRfC3 * z2) + kRfC1 * z3;
+    const double bz = (kRfB1 * z0 - kRfB2 * z1) + kRfB1 * z3;
+    const double hx = x2 + x1, hy = y1 + y2, hz = z1 + z2;
+    const double num2 =   // twice the numerator
+        z0 * ((z3 - 3.0 * z0) + hz) + y3 * ((hy - 3.0 * y3) + y0) +
+        x2 * (((x0 - 3.0 * x2) + x1) + x3) + z1 * (((z0 - 3.0 * z1) + z2) + z3) +
+        z2 * (((z0 + z1) - 3.0 * z2) + z3) + z3 * ((z0 - 3.0 * z3) + hz) +
+        x0 * ((hx - 3.0 * x0) + x3) + x1 * (((x2 + x0) - 3.0 * x1) + x3) +
+        x3 * ((hx + x0) - 3.0 * x3) + y0 * ((y3 + hy) - 3.0 * y0) +
+        y1 * (((y3 + y0) - 3.0 * y1) + y2) + y2 * (((y3 + y0) + y1) - 3.0 * y2);
+    const double det = ((z0 - z3) * (cy * bx - by * cx) - (y0 - y3) * (cz * bx - cx * bz)) +
+                       (x0 - x3) * (by * cz - cy * bz);
+    return (-0.5 * num2) * rf_pow_m13((det * det));
+}
+
+__device__ __forceinline__ void amips_rf_jacobian_in(const double* T, double* J) {
+    const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
+    const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
+    const double dy = y0 - y3, dz = z0 - z3, dx = x0 - x3;
+    const double bx = (kRfB1 * x0 - kRfB2 * x1) + kRfB1 * x3;
+    const double by = (kRfB1 * y0 - kRfB2 * y1) + kRfB1 * y3;
+    const double bz = (kRfB1 * z0 - kRfB2 * z1) + kRfB1 * z3;
+    const double cx = ((kRfC1 * x0 - kRfC3 * x2) + kRfC1 * x1) + kRfC1 * x3;
+    const double cy = ((kRfC1 * y0 + kRfC1 * y1) - kRfC3 * y2) + kRfC1 * y3;
+    const double cz = ((kRfC1 * z1 - kRfC3 * z2) + kRfC1 * z3) + kRfC1 * z0;
+    const double czbx = cz * bx - bz * cx;
+    const double cybx = cy * bx, cxby = cx * by;
+    const double det = (czbx * dy - dz * (cybx - cxby)) - dx * (cz * by - bz * cy);
+    const double r = rf_pow_m13((det * det));
+    const double sz = kRfS2 * z1 - kRfS2 * z2, sy = kRfS2 * y1 - kRfS2 * y2;
+    const double sx = kRfS2 * x1 - kRfS2 * x2;
+    const double hx = x2 + x1, hy = y1 + y2, hz = z1 + z2;
+    const double num = 0.5 * (
+        y0 * ((y3 - 3.0 * y0) + hy) + z1 * (((z2 - 3.0 * z1) + z3) + z0) +
+        z2 * (((z1 - 3.0 * z2) + z3) + z0) + z3 * ((hz - 3.0 * z3) + z0) +
+        y3 * ((y0 - 3.0 * y3) + hy) + x2 * (((x0 - 3.0 * x2) + x1) + x3) +
+        y1 * (((y0 + y3) - 3.0 * y1) + y2) + y2 * (((y0 + y3) + y1) - 3.0 * y2) +
+        x0 * ((hx - 3.0 * x0) + x3) + x1 * (((x2 + x0) - 3.0 * x1) + x3) +
+        x3 * ((x0 + hx) - 3.0 * x3) + z0 * ((z3 + hz) - 3.0 * z0));
+    bool good;
+    const double rdet = recip_seeded(det, good);
+    const double w = div_seeded(kRf2_3 * num, det, rdet, good);
+    const double q0 = ((sz * (y3 - y0) - sy * (z3 - z0)) - bz * cy) + by * cz;
+    J[0] = -(r * ((((x2 - 3.0 * x0) + w * q0) + x1) + x3));
+    J[1] = r * ((((3.0 * y0 - y3) - y1) - y2) + w * ((czbx + dz * sx) - dx * sz));
+    J[2] = r * (((((-z1) - z2) - z3) + w * (((-(dy * sx)) - cybx) + cxby + dx * sy)) + 3.0 * z0);
+}
+
+// tiny (kRfTiny times the numerator, summed as the reference has it).
+static __device__ __noinline__ double rf_tiny(const double* T) {
+    const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
+    const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
+    const double hx = x2 + x1, hy = y1 + y2, hz = z1 + z2;
+    return 0.5 * ((kRfTiny * z0) * ((z3 - 3.0 * z0) + hz) + (kRfTiny * y0) * ((y3 - 3.0 * y0) + hy) +
+                  (kRfTiny * y1) * (((y0 - 3.0 * y1) + y2) + y3) +
+                  (kRfTiny * y2) * (((y0 + y1) - 3.0 * y2) + y3) +
+                  (kRfTiny * y3) * ((y0 - 3.0 * y3) + hy) + (kRfTiny * z3) * ((z0 - 3.0 * z3) + hz) +
+                  (kRfTiny * x2) * (((x0 - 3.0 * x2) + x1) + x3) +
+                  (kRfTiny * z1) * (((z0 + z3) - 3.0 * z1) + z2) +
+                  (kRfTiny * z2) * (((z0 + z3) + z1) - 3.0 * z2) +
+                  (kRfTiny * x0) * ((hx - 3.0 * x0) + x3) +
+                  (kRfTiny * x1) * (((x2 + x0) - 3.0 * x1) + x3) +
+                  (kRfTiny * ((x0 + hx) - 3.0 * x3)) * x3);
+}
+// fl(a - fl(tiny z)) for tiny = tf to 3e-7: a correction of a few units.
+__device__ __forceinline__ double sub_tiny(double a, float tf, double z, bool ok,
+                                           const double* T) {
+    const int ea = exponent_field(a), ez = exponent_field(z);
+    ok = ok && ea > 948 && ea < 1200 && ez < 1100;
+    const float zs = ez < 920 ? 0.0f : significand32(z) * __uint_as_float((uint32_t)(ez - 896) << 23);
+    const uint32_t sgn = ((uint32_t)__double2hiint(a) ^ (uint32_t)__double2hiint(z)) & 0x80000000u;
+    const float mag = tf * zs * __uint_as_float((uint32_t)(1202 - max(948, min(ea, 1200))) << 23);
+    const float g = -__uint_as_float(__float_as_uint(mag) ^ sgn);
+    const double out = add_units(a, g, 0.0f, fmaf(fabsf(g), 1e-6f, 1e-6f), ok);
+    if (ok) return out;
+    double C[12];
+    for (int k = 0; k < 12; ++k) C[k] = T[k];
+    return a - rf_tiny(C) * z;
+}
+
+__device__ __forceinline__ void amips_rf_hessian_in(const double* T, int ce, double* H) {
+    const double x0 = T[0], y0 = T[1], z0 = T[2], x1 = T[3], y1 = T[4], z1 = T[5];
+    const double x2 = T[6], y2 = T[7], z2 = T[8], x3 = T[9], y3 = T[10], z3 = T[11];
+    const double dz = z0 - z3, dx = x0 - x3, dy = y0 - y3;
+    const double bx = (kRfB1 * x0 - kRfB2 * x1) + kRfB1 * x3;
+    const double by = (kRfB1 * y0 - kRfB2 * y1) + kRfB1 * y3;
+    const double bz = (kRfB1 * z0 - kRfB2 * z1) + kRfB1 * z3;
+    const double cx = ((kRfC1 * x0 + kRfC1 * x1) - kRfC3 * x2) + kRfC1 * x3;
+    const double cy = ((kRfC1 * y0 + kRfC1 * y1) - kRfC3 * y2) + kRfC1 * y3;
+    const double cz = ((kRfC1 * z0 + kRfC1 * z1) - kRfC3 * z2) + kRfC1 * z3;
+    const double bxcy = bx * cy, bycx = by * cx;
+    const double mx = dz * (bxcy - bycx);
+    const double bycz = by * cz, cybz = cy * bz;
+    const double myz = bycz - cybz;
+    const double my = dx * myz;
+    const double bxcz = bx * cz, cxbz = cx * bz;
+    const double mxz = bxcz - cxbz;
+    const double mz = dy * mxz;
+    const double det = (mx + my) - mz;
+    const double det2 = (det * det);
+    const double r = rf_pow_m13(det2);
+    const double lx = ((x2 - 3.0 * x0) + x1) + x3;
+    const double sy = kRfS2 * y1 - kRfS2 * y2;
+    const double dzsy = dz * sy;
+    const double sz = kRfS2 * z1 - kRfS2 * z2;
+    const double dysz = dy * sz;
+    const double u = (myz + dzsy) - dysz;
+    bool good, good2;
+    const double rdet = recip_seeded(det, good), rdet2 = recip_seeded(det2, good2);
+    const double k43 = div_seeded(kRf4_3, det, rdet, good);
+    const double idet2 = div_seeded(1.0, det2, rdet2, good2);
+    // twice the reference's linear forms
+    const double hx = x2 + x1;
+    const double Lx0 = (hx - 3.0 * x0) + x3;
+    const double Lx3 = (x0 + hx) - 3.0 * x3;
+    const double Lx2 = ((x0 - 3.0 * x2) + x1) + x3;
+    const double Lx1 = ((x2 + x0) - 3.0 * x1) + x3;
+    const double hy = y1 + y2;
+    const double Ly0 = (y3 - 3.0 * y0) + hy;
+    const double Ly3 = (y0 - 3.0 * y3) + hy;
+    const double Ly2 = ((y0 + y1) - 3.0 * y2) + y3;
+    const double Ly1 = ((y0 - 3.0 * y1) + y2) + y3;
+    const double hz = z1 + z2;
+    const double Lz0 = (z3 - 3.0 * z0) + hz;
+    const double Lz3 = (z0 - 3.0 * z3) + hz;
+    const double Lz2 = ((z0 + z3) + z1) - 3.0 * z2;
+    const double Lz1 = ((z0 + z3) - 3.0 * z1) + z2;
+    const double num = 0.5 * (z0 * Lz0 + y0 * Ly0 + y1 * Ly1 + y2 * Ly2 + y3 * Ly3 + z3 * Lz3 +
+                              x2 * Lx2 + z1 * Lz1 + z2 * Lz2 + x0 * Lx0 + x1 * Lx1 + Lx3 * x3);
+    // The reference's residue term tiny = kRfTiny num, but for the rounding of
+    // its own sum: within 4.2e-14 M / sqrt|num| relative (15 roundings of terms
+    // that add up to at most 18 M max|edge| <= 25 M sqrt|num|, M the largest
+    // |coordinate|), 7e-8 for |num| >= 4e-13 M^2.  It changes H by some units of
+    // the last place, so binary32 carries it (sub_tiny).
+    const float numf = d2f_rn(num);
+    const float Mf = __uint_as_float((uint32_t)max(1, min(ce - 895, 254)) << 23);
+    const bool tok = fabsf(numf) >= 4e-13f * Mf * Mf && fabsf(numf) > 1e-15f && Mf < 1e15f;
+    const float tf = 1.85037170770859e-17f * numf;
+    const double k49n = (kRf4_9 * idet2) * num;
+    const double nd = idet2 * num;
+    const double ineg = -div_seeded(1.0, det, rdet, good);
+    const double rneg = ineg * r;
+    const double sx = kRfS2 * x1 - kRfS2 * x2;
+    const double v1 = (((kRf2_3 * bx) * cz + (kRf2_3 * dz) * sx) - (kRf2_3 * cx) * bz) -
+                      (kRf2_3 * dx) * sz;
+    const double ly = ((y1 - 3.0 * y0) + y2) + y3;
+    const double ey = y3 - y0, ez = z3 - z0;
+    const double v2 = (((-kRf2_3 * sy) * ez + (kRf2_3 * sz) * ey) + (kRf2_3 * by) * cz) -
+                      (kRf2_3 * bz) * cy;
+    const double dzsx = dz * sx, dxsz = dx * sz;
+    const double p = (dzsx - dxsz) + mxz;
+    const double q = ((sz * ey - sy * ez) + by * cz) - bz * cy;
+    const double a1 = ((((kRf4_9 * p) * q) * num) * ineg + lx * v1) - ly * v2;
+    const double un = (u * num) * ineg;
+    const double v3 = (((kRf2_3 * by) * cx - (kRf2_3 * bx) * cy) + (kRf2_3 * dx) * sy) -
+                      (kRf2_3 * dy) * sx;
+    const double lz = ((z3 - 3.0 * z0) + z1) + z2;
+    const double t = ((bycx - bxcy) + dx * sy) - dy * sx;
+    const double tn = ((kRf4_9 * t) * num) * ineg;
+    const double a2 = (q * tn + v3 * lx) - lz * v2;
+    const double ex = x3 - x0;
+    const double w1 = (num * ineg) * (((ex * sz - sx * ez) + bx * cz) - cx * bz);
+    const double s = ((dxsz - dzsx) - bxcz) + cxbz;
+    const double a3 = ((-p) * tn + v3 * ly) + lz * v1;
+    const double w2 = (num * ineg) * (((ex * (-sy) + sx * ey) - bx * cy) + cx * by);
+    H[0] = r * ((((lx * u) * k43 - (u * u) * k49n) + ((kRf2_3 * u) * nd) * (((cybz - bycz) - dzsy) + dysz)) + 3.0);
+    H[1] = rneg * (sub_tiny(a1, tf, z1, tok, T) + un * v1);
+    H[2] = rneg * (un * v3 + a2);
+    H[3] = rneg * (a1 + w1 * v2);
+    H[4] = r * ((((-(s * s)) * k49n + (s * k43) * ly) + (s * nd) * v1) + 3.0);
+    H[5] = rneg * (a3 - sub_tiny(v3 * w1, tf, -x1, tok, T));
+    H[6] = rneg * (sub_tiny(a2, tf, y1, tok, T) + w2 * v2);
+    H[7] = rneg * (a3 - w2 * v1);
+    H[8] = r * ((((-lz) * t) * k43 - (kRf10_9 * (t * t)) * nd) + 3.0);
+}
+
+// E (when WE), J and H (when non-null) of the reference form.  The range is
+// checked once for all three, so that they share their common terms.
+template <bool WE>
+__device__ __forceinline__ double amips_rf(const double* T, double* J, double* H) {
+    const int ce = coord_exponent(T);
+    double e = 0.0;
+    if (coords_in_range(ce)) {
+        if (WE) e = amips_rf_energy_in(T);
+        if (J) amips_rf_jacobian_in(T, J);
+        if (H) amips_rf_hessian_in(T, ce, H);
+        return e;
+    }
+    double C[12], Jc[3], Hc[9];   // copies: the calls keep no caller's array in memory
+    for (int k = 0; k < 12; ++k) C[k] = T[k];
+    if (WE) e = amips_rf_energy_plain(C);
+    if (J) {
+        amips_rf_jacobian_plain(C, Jc);
+        for (int k = 0; k < 3; ++k) J[k] = Jc[k];
+    }
+    if (H) {
+        amips_rf_hessian_plain(C, Hc);
+        for (int k = 0; k < 9; ++k) H[k] = Hc[k];
+    }
+    return e;
+}
+__device__ __forceinline__ double amips_rf_energy(const double* T) {
+    return amips_rf<true>(T, nullptr, nullptr);
+}
+
 // Energy form of the FP64 evaluations (TW_ENERGY_FORM_*): the reference form
 // (the default: agrees with the reference to its rounding) or the closed form.
 __device__ __forceinline__ double amips_energy_f(const double* T, int form) {
@@ -351,21 +699,12 @@ __device__ __forceinline__ double amips_energy_f(const double* T, int form) {
 // they come from the three separate routines, as NewtonsUpdate calls them
 // (VertexSmoother.cpp:654-672).
 __device__ __forceinline__ double amips_egh_f(const double* T, double* J, double* H, int form) {
-    if (form == TW_ENERGY_FORM_CLOSED) return amips_egh(T, J, H);
-    const double e = amips_rf_energy(T);
-    if (J) amips_rf_jacobian(T, J);
-    if (H) amips_rf_hessian(T, H);
-    return e;
+    return form == TW_ENERGY_FORM_CLOSED ? amips_egh(T, J, H) : amips_rf<true>(T, J, H);
 }
-
 // J and H alone, the operations of amips_egh_f.
 __device__ __forceinline__ void amips_jh_f(const double* T, double* J, double* H, int form) {
-    if (form == TW_ENERGY_FORM_CLOSED) {
-        amips_egh(T, J, H);
-    } else {
-        amips_rf_jacobian(T, J);
-        amips_rf_hessian(T, H);
-    }
+    if (form == TW_ENERGY_FORM_CLOSED) amips_egh(T, J, H);
+    else amips_rf<false>(T, J, H);
 }
 
 // ---------------------------------------------------------------------------
@@ -499,13 +838,13 @@ static __device__ __noinline__ int orient3d_exact(const double* p, const double*
     return (top > 0.0) - (top < 0.0);
 }
 
-// Returns +1 POSITIVE, 0 COPLANAR (or non-finite input), -1 NEGATIVE.
-// *exact_used is set when the filter could not decide.
-__device__ __forceinline__ int orient3d(const double* p, const double* q, const double* r,
-                                        const double* s, int* exact_used = nullptr) {
-    double ux = q[0] - p[0], uy = q[1] - p[1], uz = q[2] - p[2];
-    double vx = r[0] - p[0], vy = r[1] - p[1], vz = r[2] - p[2];
-    double wx = s[0] - p[0], wy = s[1] - p[1], wz = s[2] - p[2];
+// The sign by the binary64 filter on the differences u, v, w of the vertices
+// from p, else exactly: +1 POSITIVE, 0 COPLANAR (or non-finite input), -1
+// NEGATIVE.  *exact_used is set when the filter could not decide.
+__device__ __forceinline__ int orient3d_staged(const double* p, const double* q, const double* r,
+                                               const double* s, double ux, double uy, double uz,
+                                               double vx, double vy, double vz, double wx,
+                                               double wy, double wz, int* exact_used) {
     double vywz = vy * wz, vzwy = vz * wy;
     double vzwx = vz * wx, vxwz = vx * wz;
     double vxwy = vx * wy, vywx = vy * wx;
@@ -523,77 +862,54 @@ __device__ __forceinline__ int orient3d(const double* p, const double* q, const 
         finite_in = finite_in && isfinite(p[k]) && isfinite(q[k]) && isfinite(r[k]) && isfinite(s[k]);
     if (!finite_in) return 0;
     if (exact_used) *exact_used = 1;
-    return orient3d_exact(p, q, r, s);
+    // copies: the out-of-line call keeps no caller's array in memory
+    double a[3], b[3], c[3], d[3];
+    for (int k = 0; k < 3; ++k) {
+        a[k] = p[k];
+        b[k] = q[k];
+        c[k] = r[k];
+        d[k] = s[k];
+    }
+    return orient3d_exact(a, b, c, d);
 }
 
-// ---------------------------------------------------------------------------
-// binary32 <-> binary64 conversions in integer arithmetic.  On this GPU the
-// hardware conversions issue to the (slow) FP64 pipe; these use only the
-// integer ALU, for every class of input (normal, subnormal, zero, infinity,
-// NaN), and agree with the hardware bit for bit (tw_self_test checks it).
-// ---------------------------------------------------------------------------
-// Exact: every binary32 value is a binary64 value.
-__device__ __forceinline__ double f2d_exact(float f) {
-    uint32_t b = __float_as_uint(f);
-    uint32_t s = b & 0x80000000u;
-    uint32_t e = (b >> 23) & 0xffu;
-    uint32_t m = b & 0x7fffffu;
-    uint32_t hi, lo;
-    if (e == 0xffu) {            // inf / NaN: payload kept
-        hi = s | 0x7ff00000u | (m >> 3);
-        lo = m << 29;
-    } else if (e != 0u) {        // normal
-        hi = s | ((e + (1023u - 127u)) << 20) | (m >> 3);
-        lo = m << 29;
-    } else if (m == 0u) {        // signed zero
-        hi = s;
-        lo = 0u;
-    } else {                     // subnormal: m * 2^-149, top bit at position p
-        uint32_t p = 31u - (uint32_t)__clz(m);
-        unsigned long long mant = ((unsigned long long)m << (52u - p)) & 0x000fffffffffffffULL;
-        hi = s | ((p + 1023u - 149u) << 20) | (uint32_t)(mant >> 32);
-        lo = (uint32_t)mant;
-    }
-    return __hiloint2double((int)hi, (int)lo);
+// Orientation sign of det[d1, d2, d3] when binary32 can certify it, else 2.
+// The bound adds the rounding of the FP64 differences (3.01 u per term of the
+// permanent) to the stage-A bound (7 + 56 u) u of the binary32 evaluation.
+__device__ __forceinline__ int orient32_filter(const float* d1, const float* d2, const float* d3) {
+    float vywz = d2[1] * d3[2], vzwy = d2[2] * d3[1];
+    float vzwx = d2[2] * d3[0], vxwz = d2[0] * d3[2];
+    float vxwy = d2[0] * d3[1], vywx = d2[1] * d3[0];
+    float det = (d1[0] * (vywz - vzwy) + d1[1] * (vzwx - vxwz)) + d1[2] * (vxwy - vywx);
+    float perm = (fabsf(d1[0]) * (fabsf(vywz) + fabsf(vzwy)) +
+                  fabsf(d1[1]) * (fabsf(vzwx) + fabsf(vxwz))) +
+                 fabsf(d1[2]) * (fabsf(vxwy) + fabsf(vywx));
+    if (!(perm > 1e-30f) || !(perm < 1e30f)) return 2;
+    float bound = 11.0f * kU32 * perm;
+    if (det > bound) return 1;
+    if (-det > bound) return -1;
+    return 2;
 }
-// Round to nearest, ties to even (the IEEE default), like __double2float_rn.
-__device__ __forceinline__ float d2f_rn(double x) {
-    unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-    uint32_t s = hi & 0x80000000u;
-    uint32_t e11 = (hi >> 20) & 0x7ffu;
-    if (e11 == 0x7ffu) {                               // inf / NaN (NaN made quiet)
-        bool nan = ((hi & 0xfffffu) | lo) != 0u;
-        return __uint_as_float(s | 0x7f800000u | (nan ? 0x00400000u | ((hi & 0xfffffu) << 3) | (lo >> 29) : 0u));
-    }
-    int e = (int)e11 - 1023 + 127;
-    if (e >= 255) return __uint_as_float(s | 0x7f800000u);   // overflow: inf
-    if (e >= 1) {                                       // normal result
-        uint32_t m = ((hi & 0xfffffu) << 3) | (lo >> 29);  // top 23 mantissa bits
-        uint32_t rest = lo & 0x1fffffffu;                  // the 29 dropped bits
-        uint32_t r = ((uint32_t)e << 23) | m;
-        // a carry out of the mantissa increments the exponent (and rounds to
-        // inf at the top of the range), as round-to-nearest requires
-        r += (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) ? 1u : 0u;
-        return __uint_as_float(s | r);
-    }
-    // subnormal or zero result: value = M53 * 2^(e11 - 1075) = k * 2^-149
-    if (e11 == 0u) return __uint_as_float(s);          // double zero or subnormal
-    unsigned long long M = (b & 0x000fffffffffffffULL) | 0x0010000000000000ULL;
-    uint32_t sh = 926u - e11;                           // >= 30 here
-    if (sh > 54u) return __uint_as_float(s);            // below half the smallest subnormal
-    unsigned long long k = M >> sh;
-    unsigned long long rest = M & ((1ULL << sh) - 1ULL);
-    unsigned long long half = 1ULL << (sh - 1u);
-    k += (rest > half || (rest == half && (k & 1ULL))) ? 1ULL : 0ULL;
-    return __uint_as_float(s | (uint32_t)k);            // k = 2^23 is the smallest normal
+
+// The exact sign: a binary32 filter on the binary64 differences first (9 of
+// the binary64 filter's 38 slow instructions), then as orient3d_staged.
+__device__ __forceinline__ int orient3d(const double* p, const double* q, const double* r,
+                                        const double* s, int* exact_used = nullptr) {
+    const double u[3] = {q[0] - p[0], q[1] - p[1], q[2] - p[2]};
+    const double v[3] = {r[0] - p[0], r[1] - p[1], r[2] - p[2]};
+    const double w[3] = {s[0] - p[0], s[1] - p[1], s[2] - p[2]};
+    const float u32[3] = {d2f_rn(u[0]), d2f_rn(u[1]), d2f_rn(u[2])};
+    const float v32[3] = {d2f_rn(v[0]), d2f_rn(v[1]), d2f_rn(v[2])};
+    const float w32[3] = {d2f_rn(w[0]), d2f_rn(w[1]), d2f_rn(w[2])};
+    const int f = orient32_filter(u32, v32, w32);
+    if (f != 2) return f;
+    return orient3d_staged(p, q, r, s, u[0], u[1], u[2], v[0], v[1], v[2], w[0], w[1], w[2],
+                           exact_used);
 }
 
 // ---------------------------------------------------------------------------
 // Certified binary32 AMIPS (TW_PRECISION_FP32_CERTIFIED).
 // ---------------------------------------------------------------------------
-constexpr float kU32 = 5.9604644775390625e-08f;  // 2^-24
-
 // x^(-1/3) for a normal positive binary32 x: exponent reduction to [1,8) and
 // four Newton-Raphson steps from a linear seed; relative error below 4 u.
 __device__ __forceinline__ float icbrt32(float x) {
@@ -738,24 +1054,6 @@ __device__ __forceinline__ Energy32 amips_energy32(const float* d1, const float*
     R.ok = (aD > 1e-18f) && (aD < 1e18f) && (N > 1e-30f) && (N < 1e30f) && (R.rel <= 1e-4f);
     R.E = R.ok ? N * icbrt32(D * D) : 0.0f;
     return R;
-}
-
-// Orientation sign of det[d1, d2, d3] when binary32 can certify it, else 2.
-// The bound adds the rounding of the FP64 differences (3.01 u per term of the
-// permanent) to the stage-A bound (7 + 56 u) u of the binary32 evaluation.
-__device__ __forceinline__ int orient32_filter(const float* d1, const float* d2, const float* d3) {
-    float vywz = d2[1] * d3[2], vzwy = d2[2] * d3[1];
-    float vzwx = d2[2] * d3[0], vxwz = d2[0] * d3[2];
-    float vxwy = d2[0] * d3[1], vywx = d2[1] * d3[0];
-    float det = (d1[0] * (vywz - vzwy) + d1[1] * (vzwx - vxwz)) + d1[2] * (vxwy - vywx);
-    float perm = (fabsf(d1[0]) * (fabsf(vywz) + fabsf(vzwy)) +
-                  fabsf(d1[1]) * (fabsf(vzwx) + fabsf(vxwz))) +
-                 fabsf(d1[2]) * (fabsf(vxwy) + fabsf(vywx));
-    if (!(perm > 1e-30f) || !(perm < 1e30f)) return 2;
-    float bound = 11.0f * kU32 * perm;
-    if (det > bound) return 1;
-    if (-det > bound) return -1;
-    return 2;
 }
 
 // calTetQuality_AMIPS (LocalOperations.cpp:862-884) sentinel rule.

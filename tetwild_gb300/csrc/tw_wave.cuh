@@ -14,7 +14,8 @@
 // takes the next star.  A fixed group of lanes per star, as before, left a
 // third of the lanes idle on the last tets of each star, summed all 13
 // components on every lane and solved on every lane: 2 x the binary64
-// instructions (20k stars to convergence: 5.5 ms, now 3.2).
+// instructions (20k stars to convergence: 5.5 ms, here 3.2, 2.9 with the
+// shorter evaluations of tw_exact.cuh).
 //
 // CERT (TW_PRECISION_FP32_CERTIFIED): inversion signs come from the certified
 // binary32 filter first, and the star energies, which only decide whether a
@@ -22,7 +23,7 @@
 // decide, the star's energies are evaluated in binary64 (kEnergyOld /
 // kEnergyNew).  J, H and every position stay binary64, so the results are the
 // same bit for bit.  The first stage of the 200k-star pass (one step): 14.6 ms
-// with a group of lanes per star, 6.6 here.
+// with a group of lanes per star, 5.9 here.
 #pragma once
 
 enum WaveState : int {
