@@ -930,7 +930,7 @@ void smooth_launch(tw_ctx* c, const int32_t* off, const int32_t* tets, const uin
     launch_smooth_project(c->surf[TW_SURFACE_INPUT], c->surf[TW_SURFACE_BOUNDARY], c->eps2, kinds,
                           nstars,
                           status, S.pnew, c->counters, c->stream);
-    launch_smooth_stage2(c->newton_shape, c->vx, c->vy, c->vz, off, tets, ff, cen, nstars, S.pnew,
+    launch_smooth_stage2(c->newton_shape, c->precision, c->vx, c->vy, c->vz, off, tets, ff, cen, nstars, S.pnew,
                          status, S.faces, S.face_count, S.face_cap, S.face_base, S.face_cnt,
                          c->counters, c->stream, c->energy_form);
     launch_env_faces_dev(c->surf[TW_SURFACE_INPUT], S.faces, S.face_count, S.face_cap, c->eps2,
@@ -1222,7 +1222,7 @@ int tw_collapse_check(tw_ctx* c, const int32_t* v12, const uint8_t* flags, const
     launch_collapse_points(c->surf[TW_SURFACE_INPUT], c->surf[TW_SURFACE_BOUNDARY], c->eps2,
                            c->precision, c->vx, c->vy, c->vz, dv, dfl, n, dst, ddeg, c->counters,
                            c->stream);
-    launch_collapse_stage(c->newton_shape, c->vx, c->vy, c->vz, doff, dt, dff, dv, dfl, ddeg, n,
+    launch_collapse_stage(c->newton_shape, c->precision, c->vx, c->vy, c->vz, doff, dt, dff, dv, dfl, ddeg, n,
                           check_quality, soft_energy, dst, S.faces, S.face_count, S.face_cap,
                           S.face_base, S.face_cnt, c->counters, c->stream, c->energy_form);
     if (any_surface)

@@ -175,6 +175,49 @@ __device__ __forceinline__ int facet_classify(const FacetCull* __restrict__ cull
                               __ldg(w + 5), w6, q);
 }
 
+// Certified bounds L2 <= d^2 <= U2 of the distance from the point to facet f
+// (0 and infinity for a facet without a record).
+__device__ __forceinline__ void facet_bounds(const FacetCull* __restrict__ cull, int32_t f,
+                                             const CertQuery& q, float& L2, float& U2) {
+    const float4* w = reinterpret_cast<const float4*>(cull + f);
+    const float4 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3),
+                 w4 = __ldg(w + 4), w5 = __ldg(w + 5), w6 = __ldg(w + 6);
+    L2 = 0.0f;
+    U2 = __int_as_float(0x7f800000);
+    if (__float_as_uint(w6.w) == 0u) return;
+    const float rx = (q.ph[0] - w0.x) + (q.pl[0] - w0.w);
+    const float ry = (q.ph[1] - w0.y) + (q.pl[1] - w1.x);
+    const float rz = (q.ph[2] - w0.z) + (q.pl[2] - w1.y);
+    const float R1 = fabsf(rx) + fabsf(ry) + fabsf(rz);
+    const float n0 = w1.z, n1 = w1.w, n2 = w2.x;
+    const float ne[3][3] = {{w2.y, w2.z, w2.w}, {w3.x, w3.y, w3.z}, {w3.w, w4.x, w4.y}};
+    const float c[3] = {w4.z, w4.w, w5.x}, o[3] = {w5.y, w5.z, w5.w}, len[3] = {w6.x, w6.y, w6.z};
+    const float h = fabsf(fmaf(n2, rz, fmaf(n1, ry, n0 * rx)));
+    const float dh = fmaf(8.0f * kUf, R1, q.Mu2);
+    const float hlo = fmaxf(h - dh, 0.0f), hhi = h + dh;
+    float sm = 0.0f;
+    bool crossed = false;
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+        const float s = fmaf(ne[e][2], rz, fmaf(ne[e][1], ry, ne[e][0] * rx)) - c[e];
+        const float ds = fmaf(10.0f * kUf, R1 + fabsf(c[e]), q.Mu2);
+        sm = fmaxf(sm, s - ds);
+        if (!(s + ds >= 0.0f)) continue;
+        crossed = true;
+        const float t0 = fmaf(n1, ne[e][2], -n2 * ne[e][1]);
+        const float t1 = fmaf(n2, ne[e][0], -n0 * ne[e][2]);
+        const float t2 = fmaf(n0, ne[e][1], -n1 * ne[e][0]);
+        const float tau = fmaf(t2, rz, fmaf(t1, ry, t0 * rx)) - o[e];
+        const float dtau = fmaf(12.0f * kUf, R1 + fabsf(o[e]), q.Mu2);
+        const float xhi = fmaxf(fmaxf(-tau, tau - len[e]), 0.0f) +
+                          fmaf(2.0f * kUf, fabsf(tau) + len[e], dtau);
+        const float shi = fabsf(s) + ds;
+        U2 = fminf(U2, fmaf(hhi, hhi, fmaf(shi, shi, xhi * xhi)));
+    }
+    if (!crossed) U2 = hhi * hhi;
+    L2 = fmaf(hlo, hlo, sm * sm);
+}
+
 // The certified test of one leaf: FP32 classification, FP64 in the band.
 __device__ __forceinline__ bool cert_leaf_within(const FacetCull* __restrict__ cull,
                                                  const double* __restrict__ tri, int32_t lf,

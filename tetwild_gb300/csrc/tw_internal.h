@@ -316,7 +316,7 @@ void launch_smooth_stage1(int shape, int precision, const double* vx, const doub
                           const int32_t* centers, const uint8_t* kinds, int32_t nstars,
                           int max_step, int max_it, double* out, double* pnew, uint8_t* status,
                           cudaStream_t s, int form = TW_ENERGY_FORM_REFERENCE);
-void launch_smooth_stage2(int shape, const double* vx, const double* vy, const double* vz,
+void launch_smooth_stage2(int shape, int precision, const double* vx, const double* vy, const double* vz,
                           const int32_t* star_off, const int32_t* tets, const uint8_t* face_flags,
                           const int32_t* centers, int32_t nstars, const double* pnew,
                           uint8_t* status, double* faces, unsigned long long* face_count,
@@ -352,7 +352,7 @@ void launch_collapse_points(const Surface& Sin, const Surface& Sb, double eps2, 
                             const double* vx, const double* vy, const double* vz,
                             const int32_t* v12, const uint8_t* flags, int32_t n, uint8_t* status,
                             uint8_t* degenerate, unsigned long long* counters, cudaStream_t s);
-void launch_collapse_stage(int shape, const double* vx, const double* vy, const double* vz,
+void launch_collapse_stage(int shape, int precision, const double* vx, const double* vy, const double* vz,
                            const int32_t* off, const int32_t* tets, const uint8_t* face_flags,
                            const int32_t* v12, const uint8_t* flags, const uint8_t* degenerate,
                            int32_t n, int check_quality, double soft_energy, uint8_t* status,

@@ -20,7 +20,9 @@ namespace tw {
 
 #include "tw_wave.cuh"
 
-template <int G>
+// CERT: signs and the largest qualities are compared as certified binary32
+// intervals first, in binary64 where those overlap (the same decisions).
+template <int G, bool CERT>
 __global__ void __launch_bounds__(256) k_smooth_stage2(
     const double* __restrict__ vx, const double* __restrict__ vy, const double* __restrict__ vz,
     const int32_t* __restrict__ star_off, const int4* __restrict__ tets,
@@ -46,21 +48,42 @@ __global__ void __launch_bounds__(256) k_smooth_stage2(
             continue;
         }
         // max calTetQuality before and after (:379-386); max is exact in any order
-        double old_max = 0.0, new_max = 0.0;
-        for (int c0 = gl; c0 < nt; c0 += G) {
-            double T[12];
-            int4 tv = tet_at(S, c0);
-            gather_tet(S, tv, 0, p0, T);
-            old_max = fmax(old_max, positive_tet_quality(T, S.form));
-            gather_tet(S, tv, 0, p, T);
-            new_max = fmax(new_max, positive_tet_quality(T, S.form));
+        int better = -1;   // not known yet
+        if (CERT) {
+            MaxBounds o, m;
+            for (int c0 = gl; c0 < nt; c0 += G) {
+                const int4 tv = tet_at(S, c0);
+                double T[12];
+                float d1[3], d2[3], d3[3];
+                gather_tet(S, tv, 0, p0, T);
+                float M = tet_diffs32(T, d1, d2, d3);
+                o.add_positive(d1, d2, d3, M);
+                gather_tet(S, tv, 0, p, T);
+                M = tet_diffs32(T, d1, d2, d3);
+                m.add_positive(d1, d2, d3, M);
+            }
+            o.join<G>(gm);
+            m.join<G>(gm);
+            if (o.sure && m.sure) better = m.hi < o.lo ? 1 : m.lo > o.hi ? 0 : -1;
         }
+        if (better < 0) {
+            double old_max = 0.0, new_max = 0.0;
+            for (int c0 = gl; c0 < nt; c0 += G) {
+                double T[12];
+                int4 tv = tet_at(S, c0);
+                gather_tet(S, tv, 0, p0, T);
+                old_max = fmax(old_max, positive_tet_quality(T, S.form));
+                gather_tet(S, tv, 0, p, T);
+                new_max = fmax(new_max, positive_tet_quality(T, S.form));
+            }
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {
-            old_max = fmax(old_max, __shfl_xor_sync(gm, old_max, o, G));
-            new_max = fmax(new_max, __shfl_xor_sync(gm, new_max, o, G));
+            for (int o = G / 2; o > 0; o >>= 1) {
+                old_max = fmax(old_max, __shfl_xor_sync(gm, old_max, o, G));
+                new_max = fmax(new_max, __shfl_xor_sync(gm, new_max, o, G));
+            }
+            better = new_max < old_max;
         }
-        if (!(new_max < old_max)) {
+        if (!better) {
             if (gl == 0) status[sid] = TW_SMOOTH_REJECT_QUALITY;
             continue;
         }
@@ -132,7 +155,7 @@ __device__ __forceinline__ bool tet_has(int4 tv, int32_t v) {
     return tv.x == v || tv.y == v || tv.z == v || tv.w == v;
 }
 
-template <int G>
+template <int G, bool CERT>
 __global__ void __launch_bounds__(256) k_collapse_stage(
     const double* __restrict__ vx, const double* __restrict__ vy, const double* __restrict__ vz,
     const int32_t* __restrict__ off, const int4* __restrict__ tets,
@@ -169,27 +192,61 @@ __global__ void __launch_bounds__(256) k_collapse_stage(
             if (gl == 0) status[e] = 1;  // FLIP
             continue;
         }
-        // quality (:390-415): max over the old tets (stored quality) and the new
-        if (check_quality) {
-            double old_max = 0.0, new_max = 0.0;
-            for (int c0 = gl; c0 < nt; c0 += G) {
-                const int4 tv = tet_at(S, c0);
-                double T[12];
-                gather_tet(S, tv, 0, p1, T);
-                old_max = fmax(old_max, quality_from(orient3d(T, T + 3, T + 6, T + 9),
-                                                     amips_energy_f(T, S.form)));
-                if (tet_has(tv, v2)) continue;
-                gather_tet(S, tv, 0, p2, T);
-                new_max = fmax(new_max, positive_tet_quality(T, S.form));
+        // quality (:390-415): max over the old tets (stored quality, or the soft
+        // bound) and the new; an unrounded v1 or a degenerate edge passes
+        if (check_quality && !deg && !(fl & TW_CV_V1_UNROUNDED)) {
+            const bool soft = soft_energy >= 0.0;
+            int worse = -1;   // not known yet
+            if (CERT) {
+                MaxBounds o, m;
+                for (int c0 = gl; c0 < nt; c0 += G) {
+                    const int4 tv = tet_at(S, c0);
+                    double T[12];
+                    float d1[3], d2[3], d3[3];
+                    if (!soft) {
+                        gather_tet(S, tv, 0, p1, T);
+                        const float M = tet_diffs32(T, d1, d2, d3);
+                        int ori = orient32_filter(d1, d2, d3);
+                        if (ori == 2) ori = orient3d(T, T + 3, T + 6, T + 9);
+                        if (ori == 1) o.add_positive(d1, d2, d3, M);
+                        else o.add_sentinel();
+                    }
+                    if (tet_has(tv, v2)) continue;
+                    gather_tet(S, tv, 0, p2, T);
+                    const float M = tet_diffs32(T, d1, d2, d3);
+                    m.add_positive(d1, d2, d3, M);
+                }
+                o.join<G>(gm);
+                m.join<G>(gm);
+                if (soft) {
+                    o.lo = __double2float_rd(soft_energy);
+                    o.hi = __double2float_ru(soft_energy);
+                }
+                if (o.sure && m.sure) worse = m.hi < o.lo ? 0 : m.lo > o.hi ? 1 : -1;
             }
+            if (worse < 0) {
+                double old_max = 0.0, new_max = 0.0;
+                for (int c0 = gl; c0 < nt; c0 += G) {
+                    const int4 tv = tet_at(S, c0);
+                    double T[12];
+                    if (!soft) {
+                        gather_tet(S, tv, 0, p1, T);
+                        old_max = fmax(old_max, quality_from(orient3d(T, T + 3, T + 6, T + 9),
+                                                             amips_energy_f(T, S.form)));
+                    }
+                    if (tet_has(tv, v2)) continue;
+                    gather_tet(S, tv, 0, p2, T);
+                    new_max = fmax(new_max, positive_tet_quality(T, S.form));
+                }
 #pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) {
-                old_max = fmax(old_max, __shfl_xor_sync(gm, old_max, o, G));
-                new_max = fmax(new_max, __shfl_xor_sync(gm, new_max, o, G));
+                for (int o = G / 2; o > 0; o >>= 1) {
+                    old_max = fmax(old_max, __shfl_xor_sync(gm, old_max, o, G));
+                    new_max = fmax(new_max, __shfl_xor_sync(gm, new_max, o, G));
+                }
+                if (soft) old_max = soft_energy;
+                worse = !(new_max <= old_max);
             }
-            if (soft_energy >= 0.0) old_max = soft_energy;
-            if (fl & TW_CV_V1_UNROUNDED) new_max = 0.0;
-            if (!deg && !(new_max <= old_max)) {
+            if (worse) {
                 if (gl == 0) status[e] = 2;  // QUALITY
                 continue;
             }
@@ -354,29 +411,27 @@ void launch_smooth_stage1(int shape, int precision, const double* vx, const doub
     else launch_wave<true, false>(shape, A, s);
 }
 
-void launch_smooth_stage2(int shape, const double* vx, const double* vy, const double* vz,
-                          const int32_t* star_off, const int32_t* tets, const uint8_t* face_flags,
-                          const int32_t* centers, int32_t nstars, const double* pnew,
-                          uint8_t* status, double* faces, unsigned long long* face_count,
-                          int64_t face_cap, int32_t* face_base, int32_t* face_cnt,
-                          unsigned long long* counters, cudaStream_t s, int form) {
+void launch_smooth_stage2(int shape, int precision, const double* vx, const double* vy,
+                          const double* vz, const int32_t* star_off, const int32_t* tets,
+                          const uint8_t* face_flags, const int32_t* centers, int32_t nstars,
+                          const double* pnew, uint8_t* status, double* faces,
+                          unsigned long long* face_count, int64_t face_cap, int32_t* face_base,
+                          int32_t* face_cnt, unsigned long long* counters, cudaStream_t s,
+                          int form) {
     if (nstars <= 0) return;
     int block;
     const int G = smooth_group(shape, &block);
     const int grid = grid_for((int64_t)nstars * G, block, 2048 / block);
     const int4* t4 = reinterpret_cast<const int4*>(tets);
-    if (G == 8)
-        k_smooth_stage2<8><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, face_flags, centers,
-                                                  nstars, pnew, status, faces, face_count, face_cap,
-                                                  face_base, face_cnt, counters, form);
-    else if (G == 16)
-        k_smooth_stage2<16><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, face_flags, centers,
-                                                   nstars, pnew, status, faces, face_count, face_cap,
-                                                   face_base, face_cnt, counters, form);
-    else
-        k_smooth_stage2<32><<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, face_flags, centers,
-                                                   nstars, pnew, status, faces, face_count, face_cap,
-                                                   face_base, face_cnt, counters, form);
+    const bool cert = precision == TW_PRECISION_FP32_CERTIFIED;
+    auto go = [&](auto kernel) {
+        kernel<<<grid, block, 0, s>>>(vx, vy, vz, star_off, t4, face_flags, centers, nstars, pnew,
+                                      status, faces, face_count, face_cap, face_base, face_cnt,
+                                      counters, form);
+    };
+    if (G == 8) cert ? go(k_smooth_stage2<8, true>) : go(k_smooth_stage2<8, false>);
+    else if (G == 16) cert ? go(k_smooth_stage2<16, true>) : go(k_smooth_stage2<16, false>);
+    else cert ? go(k_smooth_stage2<32, true>) : go(k_smooth_stage2<32, false>);
 }
 
 void launch_smooth_finalize(int32_t nstars, const int32_t* face_base, const int32_t* face_cnt,
@@ -388,28 +443,28 @@ void launch_smooth_finalize(int32_t nstars, const int32_t* face_base, const int3
                                                                    face_out, pnew, out, status);
 }
 
-void launch_collapse_stage(int shape, const double* vx, const double* vy, const double* vz,
-                           const int32_t* off, const int32_t* tets, const uint8_t* face_flags,
-                           const int32_t* v12, const uint8_t* flags, const uint8_t* degenerate,
-                           int32_t n, int check_quality, double soft_energy, uint8_t* status,
-                           double* faces, unsigned long long* face_count, int64_t face_cap,
-                           int32_t* face_base, int32_t* face_cnt, unsigned long long* counters,
-                           cudaStream_t s, int form) {
+void launch_collapse_stage(int shape, int precision, const double* vx, const double* vy,
+                           const double* vz, const int32_t* off, const int32_t* tets,
+                           const uint8_t* face_flags, const int32_t* v12, const uint8_t* flags,
+                           const uint8_t* degenerate, int32_t n, int check_quality,
+                           double soft_energy, uint8_t* status, double* faces,
+                           unsigned long long* face_count, int64_t face_cap, int32_t* face_base,
+                           int32_t* face_cnt, unsigned long long* counters, cudaStream_t s,
+                           int form) {
     if (n <= 0) return;
     int block;
     const int G = smooth_group(shape, &block);
     const int grid = grid_for((int64_t)n * G, block, 2048 / block);
     const int4* t4 = reinterpret_cast<const int4*>(tets);
-#define TW_COLLAPSE_ARGS                                                                      \
-    vx, vy, vz, off, t4, face_flags, v12, flags, degenerate, n, check_quality, soft_energy, status, \
-        faces, face_count, face_cap, face_base, face_cnt, counters, form
-    if (G == 8)
-        k_collapse_stage<8><<<grid, block, 0, s>>>(TW_COLLAPSE_ARGS);
-    else if (G == 16)
-        k_collapse_stage<16><<<grid, block, 0, s>>>(TW_COLLAPSE_ARGS);
-    else
-        k_collapse_stage<32><<<grid, block, 0, s>>>(TW_COLLAPSE_ARGS);
-#undef TW_COLLAPSE_ARGS
+    const bool cert = precision == TW_PRECISION_FP32_CERTIFIED;
+    auto go = [&](auto kernel) {
+        kernel<<<grid, block, 0, s>>>(vx, vy, vz, off, t4, face_flags, v12, flags, degenerate, n,
+                                      check_quality, soft_energy, status, faces, face_count,
+                                      face_cap, face_base, face_cnt, counters, form);
+    };
+    if (G == 8) cert ? go(k_collapse_stage<8, true>) : go(k_collapse_stage<8, false>);
+    else if (G == 16) cert ? go(k_collapse_stage<16, true>) : go(k_collapse_stage<16, false>);
+    else cert ? go(k_collapse_stage<32, true>) : go(k_collapse_stage<32, false>);
 }
 
 void launch_collapse_finalize(int32_t n, const int32_t* face_base, const int32_t* face_cnt,

@@ -178,4 +178,46 @@ __device__ __forceinline__ bool first_surface_face(const StarView& S, const uint
     return true;
 }
 
+// Differences of the tet's vertices from the first, and a power of two above
+// every coordinate's magnitude.
+__device__ __forceinline__ float tet_diffs32(const double* T, float* d1, float* d2, float* d3) {
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) m = max(m, __double2hiint(T[k]) & 0x7fffffff);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        d1[k] = d2f_rn(T[3 + k] - T[k]);
+        d2[k] = d2f_rn(T[6 + k] - T[k]);
+        d3[k] = d2f_rn(T[9 + k] - T[k]);
+    }
+    const int e = (m >> 20) - 1023 + 128;   // of 2^(exponent + 1)
+    return e <= 0 ? 1.17549435e-38f : e >= 255 ? __int_as_float(0x7f800000) : __int_as_float(e << 23);
+}
+
+// Bounds of the largest quality over the tets a lane of a group has seen
+// (certified binary32 energies); sure: every tet had one.
+struct MaxBounds {
+    float lo = 0.0f, hi = 0.0f;
+    bool sure = true;
+    __device__ __forceinline__ void add_positive(const float* d1, const float* d2,
+                                                 const float* d3, float M) {
+        const Energy32 r = amips_energy32(d1, d2, d3, M);
+        sure = sure && r.ok && r.E < 1e30f;
+        lo = fmaxf(lo, __fmul_rd(r.E, 1.0f - r.rel));
+        hi = fmaxf(hi, __fmul_ru(r.E, 1.0f + r.rel));
+    }
+    __device__ __forceinline__ void add_sentinel() {   // kMaxEnergy, above every energy here
+        lo = hi = 3e38f;
+    }
+    template <int G>
+    __device__ __forceinline__ void join(unsigned gm) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            lo = fmaxf(lo, __shfl_xor_sync(gm, lo, o, G));
+            hi = fmaxf(hi, __shfl_xor_sync(gm, hi, o, G));
+        }
+        sure = __all_sync(gm, sure);
+    }
+};
+
 }  // namespace tw

@@ -70,22 +70,6 @@ struct WaveArgs {
     uint8_t* status;           // smoothing: the state; else moved
 };
 
-// Differences of the tet's vertices from the first, and a power of two above
-// every coordinate's magnitude.
-__device__ __forceinline__ float tet_diffs32(const double* T, float* d1, float* d2, float* d3) {
-    int m = 0;
-#pragma unroll
-    for (int k = 0; k < 12; ++k) m = max(m, __double2hiint(T[k]) & 0x7fffffff);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        d1[k] = d2f_rn(T[3 + k] - T[k]);
-        d2[k] = d2f_rn(T[6 + k] - T[k]);
-        d3[k] = d2f_rn(T[9 + k] - T[k]);
-    }
-    const int e = (m >> 20) - 1023 + 128;   // of 2^(exponent + 1)
-    return e <= 0 ? 1.17549435e-38f : e >= 255 ? __int_as_float(0x7f800000) : __int_as_float(e << 23);
-}
-
 template <bool SMOOTH, bool CERT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_newton_wave(WaveArgs A) {
     __shared__ WaveShared<BLOCK> W;
