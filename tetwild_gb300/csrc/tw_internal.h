@@ -115,6 +115,9 @@ struct Surface {
     double scale = 0.0;         // max |coordinate| over the surface
     double lo[3] = {0, 0, 0};   // box of the facet centroids (Morton grid of the tree;
     double hi[3] = {0, 0, 0};   // query points are ordered on the same grid)
+    double box_lo[3] = {0, 0, 0};   // box of the facets
+    double box_hi[3] = {0, 0, 0};
+    double mean_extent = 0.0;   // mean over facets of the largest extent of their box
     size_t bytes = 0;
     EnvGrid grid;
 };

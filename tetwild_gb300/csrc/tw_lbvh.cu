@@ -16,6 +16,8 @@
 // traversal step is one line of L2/HBM traffic.
 #include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
+
 #include "tw_device.cuh"
 #include "tw_internal.h"
 
@@ -43,37 +45,71 @@ __global__ void k_gather_tris(const double* __restrict__ V, int32_t nv,
     for (int k = 0; k < 3; ++k) cen[3 * (int64_t)f + k] = c[k] / 3.0;
 }
 
-// One block: min/max of the centroids, and max |coordinate| of the facets.
-__global__ void k_bounds(const double* __restrict__ cen, const double* __restrict__ tri,
-                         int32_t nf, double* __restrict__ out) {
-    __shared__ double red[7][1024];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    double sc = 0.0;
-    for (int32_t f = threadIdx.x; f < nf; f += blockDim.x) {
-        for (int k = 0; k < 3; ++k) {
-            double x = cen[3 * (int64_t)f + k];
-            lo[k] = fmin(lo[k], x);
-            hi[k] = fmax(hi[k], x);
-        }
-        for (int k = 0; k < 9; ++k) sc = fmax(sc, fabs(tri[9 * (int64_t)f + k]));
+// Bounds of the facets: the centroids' box (0..2, 3..5), the largest
+// |coordinate| (6), the vertices' box (7..9, 10..12), and the sum over facets
+// of the largest extent (13).  In two steps, a row of kBounds values per
+// block and then one block over the rows (one block over all of 100k facets
+// took 0.44 ms, these 0.02); the sum's order is fixed by the grid.
+constexpr int kBounds = 14;
+constexpr int kBoundsBlock = 256;
+constexpr int kBoundsRows = 304;
+
+__device__ __forceinline__ double bounds_join(int k, double a, double b) {
+    return k == 13 ? a + b : (k < 3 || (k >= 7 && k < 10)) ? fmin(a, b) : fmax(a, b);
+}
+// joins the block's values (lane, then warp) into out[0 .. kBounds)
+__device__ __forceinline__ void bounds_reduce(double* v, double* __restrict__ out) {
+    __shared__ double red[kBoundsBlock / 32][kBounds];
+#pragma unroll
+    for (int k = 0; k < kBounds; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] = bounds_join(k, v[k], __shfl_xor_sync(0xffffffffu, v[k], o));
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = v[k];
     }
-    for (int k = 0; k < 3; ++k) {
-        red[k][threadIdx.x] = lo[k];
-        red[3 + k][threadIdx.x] = hi[k];
-    }
-    red[6][threadIdx.x] = sc;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            for (int k = 0; k < 3; ++k) {
-                red[k][threadIdx.x] = fmin(red[k][threadIdx.x], red[k][threadIdx.x + w]);
-                red[3 + k][threadIdx.x] = fmax(red[3 + k][threadIdx.x], red[3 + k][threadIdx.x + w]);
-            }
-            red[6][threadIdx.x] = fmax(red[6][threadIdx.x], red[6][threadIdx.x + w]);
-        }
-        __syncthreads();
+    if (threadIdx.x < kBounds) {
+        double x = red[0][threadIdx.x];
+        for (int w = 1; w < kBoundsBlock / 32; ++w) x = bounds_join(threadIdx.x, x, red[w][threadIdx.x]);
+        out[threadIdx.x] = x;
     }
-    if (threadIdx.x < 7) out[threadIdx.x] = red[threadIdx.x][0];
+}
+__device__ __forceinline__ void bounds_start(double* v) {
+#pragma unroll
+    for (int k = 0; k < kBounds; ++k)
+        v[k] = (k == 6 || k == 13) ? 0.0 : (k < 3 || (k >= 7 && k < 10)) ? INFINITY : -INFINITY;
+}
+__global__ void __launch_bounds__(kBoundsBlock) k_bounds_rows(const double* __restrict__ cen,
+                                                              const double* __restrict__ tri,
+                                                              int32_t nf, double* __restrict__ rows) {
+    double v[kBounds];
+    bounds_start(v);
+    for (int64_t f = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; f < nf;
+         f += (int64_t)gridDim.x * blockDim.x) {
+        double ext = 0.0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double x = cen[3 * f + k];
+            v[k] = fmin(v[k], x);
+            v[3 + k] = fmax(v[3 + k], x);
+            const double a = tri[9 * f + k], b = tri[9 * f + 3 + k], c = tri[9 * f + 6 + k];
+            v[6] = fmax(v[6], fmax(fabs(a), fmax(fabs(b), fabs(c))));
+            const double lo = fmin(a, fmin(b, c)), hi = fmax(a, fmax(b, c));
+            v[7 + k] = fmin(v[7 + k], lo);
+            v[10 + k] = fmax(v[10 + k], hi);
+            ext = fmax(ext, hi - lo);
+        }
+        v[13] += ext;
+    }
+    bounds_reduce(v, rows + (int64_t)blockIdx.x * kBounds);
+}
+__global__ void __launch_bounds__(kBoundsBlock) k_bounds(const double* __restrict__ rows, int nrows,
+                                                         double* __restrict__ out) {
+    double v[kBounds];
+    bounds_start(v);
+    for (int r = threadIdx.x; r < nrows; r += blockDim.x)
+#pragma unroll
+        for (int k = 0; k < kBounds; ++k) v[k] = bounds_join(k, v[k], rows[r * kBounds + k]);
+    bounds_reduce(v, out);
 }
 
 __global__ void k_morton(const double* __restrict__ cen, int32_t nf,
@@ -286,23 +322,29 @@ int build_surface(tw_ctx* c, Surface& S, const double* dV, int32_t nv, const int
     const size_t ni = n > 1 ? n - 1 : 1;
     int st = TW_OK;
     void *nodes = nullptr, *tri = nullptr, *fid = nullptr, *nodes32 = nullptr, *cull = nullptr;
-    void *tri_in = nullptr, *cen = nullptr, *codes = nullptr, *codes2 = nullptr, *ids = nullptr,
-         *ids2 = nullptr, *leafbox = nullptr, *ibox = nullptr, *ipar = nullptr, *lpar = nullptr,
-         *flags = nullptr, *bounds = nullptr, *bad = nullptr, *temp = nullptr;
     size_t temp_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                     (int32_t*)nullptr, (int32_t*)nullptr, (int)n, 0, 30, s);
+    // the temporaries share one allocation
+    void* scratch = nullptr;
+    size_t at = 0;
+    auto part = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) & ~size_t(255);
+        return o;
+    };
+    const size_t o_tri_in = part(72 * n), o_cen = part(24 * n), o_codes = part(4 * n),
+                 o_codes2 = part(4 * n), o_ids = part(4 * n), o_ids2 = part(4 * n),
+                 o_leafbox = part(48 * n), o_ibox = part(48 * ni), o_ipar = part(4 * ni),
+                 o_lpar = part(4 * n), o_flags = part(4 * ni), o_bounds = part(8 * kBounds),
+                 o_rows = part(8 * kBounds * kBoundsRows), o_bad = part(4),
+                 o_temp = part(temp_bytes + 16);
     struct A {
         void** p;
         size_t b;
     } allocs[] = {
-        {&nodes, sizeof(BvhNode) * ni}, {&tri, 72 * n},       {&fid, 4 * n},
-        {&nodes32, sizeof(BvhNode32) * ni}, {&cull, sizeof(FacetCull) * n},
-        {&tri_in, 72 * n},              {&cen, 24 * n},       {&codes, 4 * n},
-        {&codes2, 4 * n},               {&ids, 4 * n},        {&ids2, 4 * n},
-        {&leafbox, 48 * n},             {&ibox, 48 * ni},     {&ipar, 4 * ni},
-        {&lpar, 4 * n},                 {&flags, 4 * ni},     {&bounds, 8 * 8},
-        {&bad, 4},                      {&temp, temp_bytes + 16},
+        {&nodes, sizeof(BvhNode) * ni}, {&tri, 72 * n}, {&fid, 4 * n},
+        {&nodes32, sizeof(BvhNode32) * ni}, {&cull, sizeof(FacetCull) * n}, {&scratch, at},
     };
     const int nalloc = (int)(sizeof(allocs) / sizeof(allocs[0]));
     int done = 0;
@@ -310,6 +352,12 @@ int build_surface(tw_ctx* c, Surface& S, const double* dV, int32_t nv, const int
         st = dev_alloc(c, allocs[done].b, allocs[done].p);
         if (st != TW_OK) break;
     }
+    char* sc = (char*)scratch;
+    void *tri_in = sc + o_tri_in, *cen = sc + o_cen, *codes = sc + o_codes, *codes2 = sc + o_codes2,
+         *ids = sc + o_ids, *ids2 = sc + o_ids2, *leafbox = sc + o_leafbox, *ibox = sc + o_ibox,
+         *ipar = sc + o_ipar, *lpar = sc + o_lpar, *flags = sc + o_flags, *bounds = sc + o_bounds,
+         *bad = sc + o_bad, *temp = sc + o_temp;
+    double* rows = (double*)(sc + o_rows);
     if (st == TW_OK) {
         const int B = 256;
         const int G = (int)((n + B - 1) / B);
@@ -317,7 +365,10 @@ int build_surface(tw_ctx* c, Surface& S, const double* dV, int32_t nv, const int
         cudaMemsetAsync(flags, 0, 4 * ni, s);
         cudaMemsetAsync(nodes, 0, sizeof(BvhNode) * ni, s);
         k_gather_tris<<<G, B, 0, s>>>(dV, nv, dF, nf, (double*)tri_in, (double*)cen, (int*)bad);
-        k_bounds<<<1, 1024, 0, s>>>((const double*)cen, (const double*)tri_in, nf, (double*)bounds);
+        const int nrows = std::min(kBoundsRows, (int)((n + kBoundsBlock - 1) / kBoundsBlock));
+        k_bounds_rows<<<nrows, kBoundsBlock, 0, s>>>((const double*)cen, (const double*)tri_in, nf,
+                                                     rows);
+        k_bounds<<<1, kBoundsBlock, 0, s>>>(rows, nrows, (double*)bounds);
         k_morton<<<G, B, 0, s>>>((const double*)cen, nf, (const double*)bounds, (uint32_t*)codes,
                                  (int32_t*)ids);
         cub::DeviceRadixSort::SortPairs(temp, temp_bytes, (const uint32_t*)codes,
@@ -334,9 +385,9 @@ int build_surface(tw_ctx* c, Surface& S, const double* dV, int32_t nv, const int
         }
         k_facet_cull<<<G, B, 0, s>>>((const double*)tri, nf, (FacetCull*)cull);
         int hbad = 0;
-        double hb[8] = {0};
+        double hb[kBounds] = {0};
         cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s);
-        cudaMemcpyAsync(hb, bounds, 7 * sizeof(double), cudaMemcpyDeviceToHost, s);
+        cudaMemcpyAsync(hb, bounds, sizeof hb, cudaMemcpyDeviceToHost, s);
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             st = cuda_fail(c, e, "surface build");
@@ -353,7 +404,10 @@ int build_surface(tw_ctx* c, Surface& S, const double* dV, int32_t nv, const int
             for (int k = 0; k < 3; ++k) {
                 S.lo[k] = hb[k];
                 S.hi[k] = hb[3 + k];
+                S.box_lo[k] = hb[7 + k];
+                S.box_hi[k] = hb[10 + k];
             }
+            S.mean_extent = hb[13] / nf;
             S.bytes = (sizeof(BvhNode) + sizeof(BvhNode32)) * ni + (76 + sizeof(FacetCull)) * n;
             nodes = tri = fid = nodes32 = cull = nullptr;
         }
