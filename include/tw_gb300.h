@@ -60,7 +60,8 @@ extern "C" {
 #define TW_ENERGY_QUALITY 1      /* calTetQuality_AMIPS value (1e50 sentinel) */
 
 /* arithmetic modes (tw_set_precision) */
-#define TW_PRECISION_FP64 0            /* every query in binary64 (default)        */
+#define TW_PRECISION_FP64 0            /* every query in binary64 (default): what
+                                          culling leaves is evaluated in binary64  */
 #define TW_PRECISION_FP32_CERTIFIED 1  /* binary32 bulk with certified error bounds;
                                           binary64 recomputation inside the band:
                                           decisions identical to TW_PRECISION_FP64 */

@@ -399,8 +399,9 @@ __global__ void __launch_bounds__(128, MINB) k_env_points_warp(const double* __r
 // R = eps (1 + 2^-18) + 2^-17 M the cell lists cover, so both decide exactly
 // as the FP64 tree walk (some facet with computed d^2 <= eps2).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void grid_cell_range(const EnvTree& T, const CertQuery& q,
-                                                uint32_t& b, uint32_t& e) {
+template <class Tree>   // EnvTree, or the fields of it used here
+__device__ __forceinline__ void grid_cell_range(const Tree& T, const CertQuery& q, uint32_t& b,
+                                                uint32_t& e) {
     int ix[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -427,11 +428,17 @@ __device__ __forceinline__ void grid_cell_range(const EnvTree& T, const CertQuer
     }
 }
 
-__device__ __forceinline__ bool fp64_leaf_within(const double* __restrict__ tri, int32_t lf,
-                                                 const V3& p, double eps2, TravStats& st) {
+// TW_PRECISION_FP64: a facet whose certified lower bound exceeds eps is culled
+// like one whose cell or box is out of reach; every other one is evaluated in
+// binary64 (a distance costs some hundred binary64 instructions, the bound
+// none but the query's three differences): 300k points, half of them out, took
+// 0.25 ms in the test, 0.16 so.
+__device__ __forceinline__ bool fp64_leaf_within(const EnvTree& T, int32_t lf, const V3& p,
+                                                 const CertQuery& q, double eps2, TravStats& st) {
     ++st.facets;
+    if (facet_classify(T.cull, lf, q) == kFacetOut) return false;
     ++st.fp64;
-    return leaf_sqdist(tri, lf, p) <= eps2;
+    return leaf_sqdist(T.tri, lf, p) <= eps2;
 }
 
 // in iff a leaf of the point's cell tests in; every lane of the warp calls it
@@ -447,7 +454,7 @@ __device__ __forceinline__ bool grid_point_in(const EnvTree& T, const EpsParams&
     for (uint32_t k = b; k < e; ++k) {
         const int32_t next = k + 1 < e ? __ldg(T.glist + k + 1) : 0;
         if (CERT ? cert_leaf_within(T.cull, T.tri, lf, p, q, E.eps2, st)
-                 : fp64_leaf_within(T.tri, lf, p, E.eps2, st)) {
+                 : fp64_leaf_within(T, lf, p, q, E.eps2, st)) {
             in = true;
             break;
         }
@@ -557,7 +564,7 @@ __device__ __forceinline__ int bins_point_test(const EnvTree& T, const EpsParams
                 if (cls == kFacetIn) return 1;
                 band |= cls == kFacetBand;
             } else if (CERT ? cert_leaf_within(T.cull, T.tri, lf, p, q, E.eps2, st)
-                            : fp64_leaf_within(T.tri, lf, p, E.eps2, st)) {
+                            : fp64_leaf_within(T, lf, p, q, E.eps2, st)) {
                 return 1;
             }
         }
@@ -1524,7 +1531,7 @@ __device__ __forceinline__ void face_query_box(const double* t, const FaceCtx& F
 // The samples of one face with its header already computed, the whole warp:
 // 1 if some sample is out, 0 otherwise.  Samples in a cut known to be inside
 // (hull) are passed over; the others collect in the warp's queue (64 words of
-// shared memory) and are built and tested 32 at a time, so that the binary64
+// shared memory, as rows_held) and are built and tested 32 at a time, so that the binary64
 // construction and the facet tests run on full warps.  slice / slices: the
 // warp takes every slices-th step of 32 samples; stop (shared, may be null):
 // set by another warp of the face that found a sample out.  Out of line: the
@@ -1533,6 +1540,7 @@ template <bool FP32>
 __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
                                                     const double* __restrict__ tri,
                                                     const FaceCuts& hull, int k2, uint32_t* queue,
+                                                    int32_t* rows_held,
                                                     const FaceCtx& F, double sd, int slice,
                                                     int slices, const volatile int* stop,
                                                     TravStats& st, uint32_t& nq) {
@@ -1652,16 +1660,36 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
         if (drain(false, rim)) return 1;
     }
     if (drain(true, rim)) return 1;
-    // ...then the rows 1..M, 32 at a time: each lane sets up one row (start
-    // point and last index), the reference's break (the first row with
-    // distance(v0_m, v1_m) <= sd) ends the rows, and the lanes walk the chunk's
-    // samples by flat index.
-    for (int base = 1; base <= h.M; base += 32) {
-        const int m = base + lane;
+    // ...then the rows 1..M: those that meet an open cut are listed, and 32 at a
+    // time each lane sets up one (start point and last index), the reference's
+    // break (a row with distance(v0_m, v1_m) <= sd ends the rows) applies, and
+    // the lanes walk their samples by flat index.  Rows shorten by at least sd
+    // each (v0 v1 is the longest edge), so only the last two can break, which are
+    // always listed: passing over rows never passes over a break.
+    int held = 0;
+    for (int base = 1; base <= h.M || held > 0; base += 32) {
+        if (base <= h.M) {
+            const int m = base + lane;
+            const bool want = m <= h.M && (m + 1 >= h.M || hull_row_open(hull, k2, h.max_i,
+                                                                         (float)m * h.rrow));
+            const unsigned bal = __ballot_sync(0xffffffffu, want);
+            if (want) rows_held[held + __popc(bal & lt)] = m;
+            held += __popc(bal);
+            __syncwarp();
+            if (held < 32 && base + 32 <= h.M) continue;
+        }
+        const int batch = min(held, 32);
+        const int m = lane < batch ? rows_held[lane] : 0;
+        // what is left moves to the front (at most 31 entries)
+        held -= batch;
+        const int rest = lane < held ? rows_held[32 + lane] : 0;
+        __syncwarp();
+        if (lane < held) rows_held[lane] = rest;
+        __syncwarp();
         V3 v{0.0, 0.0, 0.0};
         int N1 = -1;
         double dd = 0.0;
-        const bool valid = m <= h.M;
+        const bool valid = lane < batch;
         const bool brk = valid && !sample_row(h, fv, sd, m, v, N1, dd);
         const unsigned bal = __ballot_sync(0xffffffffu, brk);
         const int first_brk = bal ? __ffs(bal) - 1 : 32;
@@ -1673,8 +1701,9 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
                 rows = N1 + 1;
             }
         }
-        // the row's first sample along v0->v1: delta_d in units of the edge
-        const float sx = d2f_rn(dd) / d2f_rn(sd) * h.r01;
+        // the row's first sample along v0->v1 (delta_d in units of the edge), and its
+        // place along v0->v2
+        const float sx = d2f_rn(dd) / d2f_rn(sd) * h.r01, sy = (float)m * h.rrow;
         int incl = rows;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -1683,7 +1712,7 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
         }
         const int excl = incl - rows;
         const int total = __shfl_sync(0xffffffffu, incl, 31);
-        auto in_row = [&](bool, uint32_t e) -> V3 {   // e: row << 26 | index (below 2^23)
+        auto in_row = [&](bool, uint32_t e) -> V3 {   // e: lane of the row << 26 | index (below 2^23)
             const int r = (int)(e >> 26);
             const V3 w{__shfl_sync(0xffffffffu, v.x, r), __shfl_sync(0xffffffffu, v.y, r),
                        __shfl_sync(0xffffffffu, v.z, r)};
@@ -1702,8 +1731,8 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
             }
             const int i = s - __shfl_sync(0xffffffffu, excl, r);
             const float x = fmaf((float)i, h.r01, __shfl_sync(0xffffffffu, sx, r));
-            push(s < total && !inside(x, (float)(base + r) * h.rrow),
-                 ((uint32_t)r << 26) | (uint32_t)i);
+            const float y = __shfl_sync(0xffffffffu, sy, r);
+            push(s < total && !inside(x, y), ((uint32_t)r << 26) | (uint32_t)i);
             if (drain(false, in_row)) return 1;
         }
         if (drain(true, in_row)) return 1;
@@ -1736,7 +1765,7 @@ __device__ __forceinline__ int face_prepare(const double* t, double sd, bool sha
 // of the sampling's 128 registers, and half of its stalls were barriers.)
 // Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
 // to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
-// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 3.0 and 0.76.
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.2 and 0.27.
 // Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
 constexpr int kFaceWarps = kFaceBlock / 32;
@@ -1745,8 +1774,9 @@ constexpr uint8_t kFaceOpen = 2;
 // pieces that a sample is worth: its binary64 distance costs that of several
 constexpr float kSampleCost32 = 0.6f, kSampleCost64 = 1.0f;
 
-// A warp takes an eighth of its share of the faces at a time (4 to 32), so
-// that small batches spread over all SMs and large ones balance.
+// The warps take tiles of faces from a counter (faces over many small facets
+// cost tens of times the others), an eighth of a warp's share each (4 to 32
+// faces), so that small batches spread over all SMs and large ones balance.
 template <bool FP32, class Ctx>
 __device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64_t n,
                                           unsigned long long* counters, Ctx ctx,
@@ -1759,8 +1789,11 @@ __device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64
     uint32_t nq = 0, nopen = 0;
     const int64_t warps = (int64_t)gridDim.x * kFaceWarps, share = n / (warps * 8);
     const int tile = (int)(share < 4 ? 4 : share > 32 ? 32 : share);
-    for (int64_t base = ((int64_t)blockIdx.x * kFaceWarps + warp) * tile; base < n;
-         base += warps * tile) {
+    for (;;) {
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(counters + kCntFaceCut, (unsigned long long)tile);
+        const int64_t base = (int64_t)__shfl_sync(0xffffffffu, at, 0);
+        if (base >= n) break;
         const int faces = (int)(n - base < tile ? n - base : tile);
         if (lane < faces) {
             FaceCtx F;
@@ -1813,6 +1846,7 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
     __shared__ SampleHeader head[kFaceBlock];
     __shared__ FaceCuts cuts[kFaceWarps];
     __shared__ uint32_t queue[kFaceWarps][64];
+    __shared__ int32_t rows_held[kFaceWarps][64];
     __shared__ uint16_t list[kFaceBlock];
     __shared__ uint8_t small[kFaceBlock], large[kFaceBlock];
     __shared__ int held, nsmall, nlarge, next, found;
@@ -1823,6 +1857,7 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     TravStats st;
     uint32_t nq = 0;
+    const int rot = (int)(blockIdx.x / ((gridDim.x + 3) / 4)) % kFaceWarps;
     const double want = fmin(fmax((double)nopen / (4.0 * gridDim.x), 2.0), (double)kFaceBlock);
     const int range = (int)fmin(want * ((double)n / (double)nopen), 4096.0) + 1;
     for (;;) {
@@ -1851,23 +1886,26 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 __syncthreads();
             }
             const int batch = before;
-            if ((int)threadIdx.x < batch) {
-                const int64_t f = base + list[threadIdx.x];
+            // one thread a face, from warp `rot` on: the blocks of an SM (a quarter of
+            // the grid apart) then put a small batch's binary64 work on different
+            // quarters of the SM
+            const int mine = (int)((threadIdx.x + kFaceBlock - 32 * rot) % kFaceBlock);
+            if (mine < batch) {
+                const int64_t f = base + list[mine];
                 FaceCtx F;
                 double sd, t[9];
                 ctx(f, F, sd);
 #pragma unroll
                 for (int k = 0; k < 9; ++k) t[k] = __ldg(tris + 9 * f + k);
-                hull_prepare(t, F.T, F.E, sd, FP32 ? kSampleCost32 : kSampleCost64,
-                             frame[threadIdx.x]);
-                SampleHeader& h = head[threadIdx.x];
-                const int state = face_prepare(t, sd, frame[threadIdx.x].k2 >= 0, h, counters);
+                hull_prepare(t, F.T, F.E, sd, FP32 ? kSampleCost32 : kSampleCost64, frame[mine]);
+                SampleHeader& h = head[mine];
+                const int state = face_prepare(t, sd, frame[mine].k2 >= 0, h, counters);
                 if (state != 2) {
                     out[f] = (uint8_t)state;
                 } else if (!h.trivial && h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace) {
-                    large[atomicAdd(&nlarge, 1)] = (uint8_t)threadIdx.x;
+                    large[atomicAdd(&nlarge, 1)] = (uint8_t)mine;
                 } else {
-                    small[atomicAdd(&nsmall, 1)] = (uint8_t)threadIdx.x;
+                    small[atomicAdd(&nsmall, 1)] = (uint8_t)mine;
                 }
             }
             __syncthreads();
@@ -1885,7 +1923,8 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                     hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[warp], 0, 1, st, nq);
                 const uint8_t o =
                     env_face_samples<FP32>(head[k], tris + 9 * f, cuts[warp], frame[k].k2,
-                                           queue[warp], F, sd, 0, 1, nullptr, st, nq);
+                                           queue[warp], rows_held[warp], F, sd, 0, 1, nullptr, st,
+                                           nq);
                 if (lane == 0) out[f] = o;
                 __syncwarp();
             }
@@ -1901,7 +1940,8 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                                    kFaceWarps, st, nq);
                 __syncthreads();
                 if (env_face_samples<FP32>(head[k], tris + 9 * f, cuts[0], frame[k].k2,
-                                           queue[warp], F, sd, warp, kFaceWarps, &found, st, nq))
+                                           queue[warp], rows_held[warp], F, sd, warp, kFaceWarps,
+                                           &found, st, nq))
                     found = 1;
                 __syncthreads();
                 if (threadIdx.x == 0) {
@@ -1951,7 +1991,7 @@ void launch_env_faces_dev(const Surface& S, const double* tris, const unsigned l
     if (n <= 0) return;
     const int block = kFaceBlock;
     const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
-    cudaMemsetAsync(counters + kCntFaceOpen, 0, 2 * sizeof(unsigned long long), s);
+    cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
     const OneFaceCtx C{FaceCtx{env_tree_for(S, eps2), eps_params(eps2), counters}, sd};
     if (precision == TW_PRECISION_FP32_CERTIFIED) {
         k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
@@ -2070,7 +2110,7 @@ void launch_env_faces_segs(const double* tris, int64_t n, const void* segs, int 
     if (n <= 0 || nsegs <= 0) return;
     const int block = kFaceBlock;
     const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
-    cudaMemsetAsync(counters + kCntFaceOpen, 0, 2 * sizeof(unsigned long long), s);
+    cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
     const SegFaceCtx C{static_cast<const EnvSeg*>(segs), nsegs, counters};
     if (precision == TW_PRECISION_FP32_CERTIFIED) {
         k_env_faces_segs_cut<true><<<gc, block, 0, s>>>(tris, n, C, out);
@@ -2200,7 +2240,7 @@ __device__ int32_t nearest_facet(const EnvTree& T, const V3& p, V3& q, double& s
 // the certified bounds L, U of the exact distances, and 16 u64 M the most a
 // computed distance is off, a leaf whose L exceeds the least U by 32 u64 M
 // cannot (2^-18 covers the binary32 sums, as in facet_classify).  Of the two to
-// three leaves of a cell one is left, mostly: 100k projections 1.36 -> 0.40 ms.
+// three leaves of a cell one is left, mostly: 100k projections 1.36 -> 0.49 ms.
 __device__ __forceinline__ bool nearest_facet_grid(const EnvTree& T, double eps2, const V3& p,
                                                    V3& q, double& sqd, int32_t& fid) {
     if (!T.gslot) return false;

@@ -188,7 +188,8 @@ constexpr int kCntBad = 7;            // host-visible argument check flag
 constexpr int kCntEnvQueries = 8;     // envelope sample/point queries
 constexpr int kCntEnvWarpFallback = 9;  // warps whose shared candidate list overflowed
 constexpr int kCntFaceOpen = 10;      // faces the cutting launch left open (zeroed before it)
-constexpr int kCntFaceNext = 11;      // and the sampling launch's next face (zeroed with it)
+constexpr int kCntFaceNext = 11;      // the sampling launch's next face, and
+constexpr int kCntFaceCut = 12;       // the cutting launch's (zeroed with it)
 // internal star states of a smoothing pass (the final ones are TW_SMOOTH_*)
 constexpr uint8_t kSmoothPendingProject = 6;   // surface star moved by Newton, not yet projected
 constexpr uint8_t kSmoothPendingEnvelope = 7;  // surface star waiting for its face tests
