@@ -206,17 +206,26 @@ struct Guard {
 
 // scratch slot layout: pipelines use slots [0, kNumPipe), their point-ordering
 // scratch [3, 3 + kNumPipe), misc uses 6, 7
+// Waits for the context's streams.  The error word comes back by a copy queued
+// behind the work, so one wait serves both (a blocking copy after three waits
+// cost a 37-point call 12 of its 48 us); the pipeline's other streams are
+// waited for only when a call has used them.
 int sync_status(tw_ctx* c, const char* where) {
-    cudaError_t e = cudaStreamSynchronize(c->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->copy_in);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(c->copy_out);
+    cudaError_t e = cudaSuccess;
+    if (c->pipes_used) {
+        e = cudaStreamSynchronize(c->copy_in);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(c->copy_out);
+        if (e == cudaSuccess) c->pipes_used = false;
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(c->host_words, c->counters + kCntError, sizeof(*c->host_words),
+                            cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, where);
     e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, where);
     // device-side error word: read and clear
-    unsigned long long err = 0;
-    e = cudaMemcpy(&err, c->counters + kCntError, sizeof(err), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(c, e, where);
+    const unsigned long long err = c->host_words[0];
     if (err) {
         cudaMemset(c->counters + kCntError, 0, sizeof(err));
         std::string m = std::string(where) + ": ";
@@ -231,7 +240,27 @@ int sync_status(tw_ctx* c, const char* where) {
 
 cudaStream_t pipe_stream(tw_ctx* c, int k) {
     if (k == 0) return c->stream;
+    c->pipes_used = true;
     return k == 1 ? c->copy_in : c->copy_out;
+}
+
+// Queues the copy of an argument check's flag to page-locked memory: valid
+// after the next sync_status.
+const int& fetch_flag(tw_ctx* c, const int* bad) {
+    cudaMemcpyAsync(c->host_words + 1, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    return *(const int*)(c->host_words + 1);
+}
+
+// Page-locked staging for the host buffers of small calls: copies to and from
+// it are queued without a wait each, and one wait ends the call.
+constexpr size_t kStageBytes = 256 << 10;
+char* host_stage(tw_ctx* c) {
+    if (!c->host_stage) {
+        void* p = nullptr;
+        if (cudaMallocHost(&p, kStageBytes) != cudaSuccess) cudaGetLastError();
+        else c->host_stage = (char*)p;
+    }
+    return c->host_stage;
 }
 
 // Device address of page-locked host memory (nullptr for pageable or device
@@ -288,6 +317,13 @@ int tw_ctx_create(int device, size_t hbm_budget_bytes, tw_ctx** out) {
         return TW_ERR_OOM;
     }
     c->counters = (unsigned long long*)cnt;
+    void* words = nullptr;
+    if (cudaMallocHost(&words, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+        cudaGetLastError();
+        tw_ctx_destroy(c);
+        return TW_ERR_OOM;
+    }
+    c->host_words = (unsigned long long*)words;
     cudaMemset(c->counters, 0, kNumCounters * sizeof(unsigned long long));
     *out = c;
     return TW_OK;
@@ -306,6 +342,8 @@ int tw_ctx_destroy(tw_ctx* c) {
     dev_free(c, c->rounded, (size_t)c->nv);
     for (auto& b : c->scratch) dev_free(c, b.ptr, b.cap);
     dev_free(c, c->counters, kNumCounters * sizeof(unsigned long long));
+    if (c->host_words) cudaFreeHost(c->host_words);
+    if (c->host_stage) cudaFreeHost(c->host_stage);
     for (auto& ev : c->ev)
         if (ev) cudaEventDestroy(ev);
     for (auto& ev : c->time_ev)
@@ -614,8 +652,7 @@ int tw_mesh_update_vertices(tw_ctx* c, const int32_t* ids, const double* xyz,
     if (rounded) cudaMemcpyAsync(drnd, rounded, (size_t)n, cudaMemcpyHostToDevice, c->stream);
     k_scatter_vertices<<<(n + 255) / 256, 256, 0, c->stream>>>(dids, dxyz, drnd, n, c->nv, c->vx,
                                                                c->vy, c->vz, c->rounded, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_mesh_update_vertices");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "vertex id out of range");
@@ -654,8 +691,7 @@ int tw_tet_quality(tw_ctx* c, const int32_t* tets, int64_t n, double* energy, ui
     cudaMemsetAsync(c->counters + 1, 0, sizeof(unsigned long long), c->stream);
     cudaMemcpyAsync(dt, tets, 16 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
     k_check_ids<<<(unsigned)((4 * n + 255) / 256), 256, 0, c->stream>>>(dt, 4 * n, c->nv, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_tet_quality");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "tet vertex id out of range");
@@ -733,6 +769,9 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
     if (c->surf[which].nf == 0) return fail(c, TW_ERR_NO_SURFACE, "no surface uploaded");
     if (n == 0) return TW_OK;
     Guard g(c->device);
+    // a small call: staged through page-locked memory, input and answer in one
+    // chunk with one wait (nullptr: the general path)
+    char* stage = 32 * (size_t)n + 64 <= kStageBytes ? host_stage(c) : nullptr;
     const int64_t C = chunk_len(n, 25, kPointChunkBytes);
     double* dP[kNumPipe];
     uint8_t* dO[kNumPipe];
@@ -745,6 +784,18 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
         dO[k] = (uint8_t*)p + 24 * (size_t)C;
         st = ensure(c, 3 + k, env_sort_scratch_bytes(C, c->sort_points), &dS[k]);
         if (st != TW_OK) return st;
+    }
+    if (stage) {
+        std::memcpy(stage, P, 24 * (size_t)n);
+        uint8_t* answer = (uint8_t*)stage + 24 * (size_t)n;
+        cudaMemcpyAsync(dP[0], stage, 24 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
+        launch_env_points(c->surf[which], dP[0], n, c->eps2, dO[0], c->precision, c->counters,
+                          c->sort_points ? dS[0] : nullptr, c->sort_points, c->point_block,
+                          c->stream);
+        cudaMemcpyAsync(answer, dO[0], (size_t)n, cudaMemcpyDeviceToHost, c->stream);
+        const int st = sync_status(c, "tw_envelope_points");
+        if (st != TW_ERR_CUDA) std::memcpy(out, answer, (size_t)n);
+        return st;
     }
     int64_t chunk = 0;
     for (int64_t i0 = 0; i0 < n; i0 += C, ++chunk) {
@@ -845,8 +896,7 @@ int tw_newton_stars(tw_ctx* c, const int32_t* star_off, const int32_t* tets, con
     if (nt > 0)
         k_check_ids<<<(unsigned)((4 * nt + 255) / 256), 256, 0, c->stream>>>(dt, 4 * nt, c->nv, bad);
     k_check_ids<<<(unsigned)((nstars + 255) / 256), 256, 0, c->stream>>>(dc, nstars, c->nv, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_newton_stars");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "star vertex id out of range");
@@ -1017,8 +1067,7 @@ int tw_smooth_stars(tw_ctx* c, const int32_t* star_off, const int32_t* tets,
     if (nt > 0)
         k_check_ids<<<(unsigned)((4 * nt + 255) / 256), 256, 0, c->stream>>>(dt, 4 * nt, c->nv, bad);
     k_check_ids<<<(unsigned)((ns + 255) / 256), 256, 0, c->stream>>>(dc, nstars, c->nv, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_smooth_stars");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "star vertex id out of range");
@@ -1059,8 +1108,7 @@ int tw_energy_stats(tw_ctx* c, const int32_t* tets, int64_t n, const uint8_t* lo
         if (locked) cudaMemcpyAsync(dl, locked, (size_t)n, cudaMemcpyHostToDevice, c->stream);
         k_check_ids<<<(unsigned)((4 * n + 255) / 256), 256, 0, c->stream>>>(dt, 4 * n, c->nv, bad);
     }
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_energy_stats");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "tet vertex id out of range");
@@ -1115,8 +1163,7 @@ int tw_dihedral_stats(tw_ctx* c, const int32_t* tets, int64_t n, const uint8_t* 
         if (locked) cudaMemcpyAsync(dl, locked, (size_t)n, cudaMemcpyHostToDevice, c->stream);
         k_check_ids<<<(unsigned)((4 * n + 255) / 256), 256, 0, c->stream>>>(dt, 4 * n, c->nv, bad);
     }
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_dihedral_stats");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "tet vertex id out of range");
@@ -1213,8 +1260,7 @@ int tw_collapse_check(tw_ctx* c, const int32_t* v12, const uint8_t* flags, const
     if (nt > 0)
         k_check_ids<<<(unsigned)((4 * nt + 255) / 256), 256, 0, c->stream>>>(dt, 4 * nt, c->nv, bad);
     k_check_ids<<<(unsigned)((2 * ns + 255) / 256), 256, 0, c->stream>>>(dv, 2 * n, c->nv, bad);
-    int hbad = 0;
-    cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+    const int& hbad = fetch_flag(c, bad);
     st = sync_status(c, "tw_collapse_check");
     if (st != TW_OK) return st;
     if (hbad) return fail(c, TW_ERR_ARG, "vertex id out of range");

@@ -172,6 +172,10 @@ struct tw_ctx {
     tw::Buffer scratch[10];
     // device counters, see the kCnt* indices below
     unsigned long long* counters = nullptr;
+    // page-locked: word 0 receives the error word, word 1 an argument check's flag
+    unsigned long long* host_words = nullptr;
+    char* host_stage = nullptr;   // page-locked staging of small calls (first use)
+    bool pipes_used = false;      // work was queued on copy_in / copy_out since the last wait
     std::string last_error;
 };
 
