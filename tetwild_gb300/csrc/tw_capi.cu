@@ -62,6 +62,19 @@ int ensure(tw_ctx* c, int slot, size_t bytes, void** out) {
     return TW_OK;
 }
 
+// Scratch for sorting n points: with room for the points' records (records set)
+// up to 128M points (32 bytes each), and without it above that, in a context
+// that is held to a memory budget, and where the device has no room for them.
+int ensure_sort(tw_ctx* c, int slot, int64_t n, void** out, bool* records) {
+    *records = n <= (int64_t(1) << 27) && !c->budget;
+    if (*records) {
+        if (ensure(c, slot, env_sort_scratch_bytes(n, c->sort_points, true), out) == TW_OK)
+            return TW_OK;
+        *records = false;
+    }
+    return ensure(c, slot, env_sort_scratch_bytes(n, c->sort_points, false), out);
+}
+
 // ---- pipe peak probes -------------------------------------------------------
 __global__ void k_fp64_probe(double* out, int iters) {
     double a0 = threadIdx.x * 1e-9, a1 = a0 + 1e-9, a2 = a0 + 2e-9, a3 = a0 + 3e-9;
@@ -742,7 +755,8 @@ int tw_envelope_points_device(tw_ctx* c, const double* P, int64_t n, int which, 
     if (c->surf[which].nf == 0) return fail(c, TW_ERR_NO_SURFACE, "no surface uploaded");
     Guard g(c->device);
     void* sort = nullptr;
-    int st = ensure(c, 3, env_sort_scratch_bytes(n, c->sort_points), &sort);
+    bool records;
+    int st = ensure_sort(c, 3, n, &sort, &records);
     if (st != TW_OK) return st;
     cudaEvent_t eb = nullptr, ee = nullptr;
     if (c->time_kernels) {
@@ -756,8 +770,8 @@ int tw_envelope_points_device(tw_ctx* c, const double* P, int64_t n, int which, 
         ++c->time_count;
     }
     launch_env_points(c->surf[which], P, n, c->eps2, out, c->precision, c->counters,
-                      c->sort_points ? sort : nullptr, c->sort_points, c->point_block, c->stream,
-                      eb, ee);
+                      c->sort_points ? sort : nullptr, c->sort_points, records, c->point_block,
+                      c->stream, eb, ee);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "tw_envelope_points_device");
     return TW_OK;
@@ -776,13 +790,14 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
     double* dP[kNumPipe];
     uint8_t* dO[kNumPipe];
     void* dS[kNumPipe];
+    bool records[kNumPipe];
     for (int k = 0; k < kNumPipe; ++k) {
         void* p;
         int st = ensure(c, k, 25 * (size_t)C + 256, &p);
         if (st != TW_OK) return st;
         dP[k] = (double*)p;
         dO[k] = (uint8_t*)p + 24 * (size_t)C;
-        st = ensure(c, 3 + k, env_sort_scratch_bytes(C, c->sort_points), &dS[k]);
+        st = ensure_sort(c, 3 + k, C, &dS[k], &records[k]);
         if (st != TW_OK) return st;
     }
     if (stage) {
@@ -790,8 +805,8 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
         uint8_t* answer = (uint8_t*)stage + 24 * (size_t)n;
         cudaMemcpyAsync(dP[0], stage, 24 * (size_t)n, cudaMemcpyHostToDevice, c->stream);
         launch_env_points(c->surf[which], dP[0], n, c->eps2, dO[0], c->precision, c->counters,
-                          c->sort_points ? dS[0] : nullptr, c->sort_points, c->point_block,
-                          c->stream);
+                          c->sort_points ? dS[0] : nullptr, c->sort_points, records[0],
+                          c->point_block, c->stream);
         cudaMemcpyAsync(answer, dO[0], (size_t)n, cudaMemcpyDeviceToHost, c->stream);
         const int st = sync_status(c, "tw_envelope_points");
         if (st != TW_ERR_CUDA) std::memcpy(out, answer, (size_t)n);
@@ -804,7 +819,8 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
         const int64_t len = std::min<int64_t>(C, n - i0);
         cudaMemcpyAsync(dP[k], P + 3 * i0, 24 * (size_t)len, cudaMemcpyHostToDevice, s);
         launch_env_points(c->surf[which], dP[k], len, c->eps2, dO[k], c->precision, c->counters,
-                          c->sort_points ? dS[k] : nullptr, c->sort_points, c->point_block, s);
+                          c->sort_points ? dS[k] : nullptr, c->sort_points, records[k],
+                          c->point_block, s);
         cudaMemcpyAsync(out + i0, dO[k], (size_t)len, cudaMemcpyDeviceToHost, s);
     }
     return sync_status(c, "tw_envelope_points");

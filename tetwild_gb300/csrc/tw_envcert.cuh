@@ -60,16 +60,26 @@ struct CertQuery {
 
 constexpr float kUf = 5.9604644775390625e-08f;  // 2^-24
 
-__device__ __forceinline__ CertQuery cert_query(const V3& p, const EpsParams& E, float scale_hi) {
-    CertQuery q;
+// p = ph + pl + an error of at most half an ulp of pl: each coordinate to
+// nearest in binary32, and what is left of it.
+__device__ __forceinline__ void cert_split(const V3& p, float* ph, float* pl) {
     const double pv[3] = {p.x, p.y, p.z};
-    float m = scale_hi;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        q.ph[k] = d2f_rn(pv[k]);
-        q.pl[k] = d2f_rn(pv[k] - f2d_exact(q.ph[k]));
-        m = fmaxf(m, fabsf(q.ph[k]));
+        ph[k] = d2f_rn(pv[k]);
+        pl[k] = d2f_rn(pv[k] - f2d_exact(ph[k]));
     }
+}
+
+__device__ __forceinline__ CertQuery cert_query_split(float ph0, float ph1, float ph2, float pl0,
+                                                      float pl1, float pl2, const EpsParams& E,
+                                                      float scale_hi) {
+    CertQuery q;
+    q.ph[0] = ph0; q.ph[1] = ph1; q.ph[2] = ph2;
+    q.pl[0] = pl0; q.pl[1] = pl1; q.pl[2] = pl2;
+    float m = scale_hi;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m = fmaxf(m, fabsf(q.ph[k]));
     const float mu = __fmul_ru(m, 1.00000012f);                          // >= max |p|, |a|
     const float slack = __fmul_ru(1.7763568394002505e-15f, mu);          // 16 u64 M
     const float tau = __fadd_ru(__fmul_ru(4.76837158203125e-07f, mu),
@@ -82,6 +92,12 @@ __device__ __forceinline__ CertQuery cert_query(const V3& p, const EpsParams& E,
     q.e2lo = el > 0.0f ? __fmul_rd(__fmul_rd(el, el), 0.999996185f) : 0.0f;  // (1 - 2^-18)
     q.Mu2 = __fmul_ru(5.684341886080802e-14f, mu);                       // 16 u^2 M
     return q;
+}
+
+__device__ __forceinline__ CertQuery cert_query(const V3& p, const EpsParams& E, float scale_hi) {
+    float ph[3], pl[3];
+    cert_split(p, ph, pl);
+    return cert_query_split(ph[0], ph[1], ph[2], pl[0], pl[1], pl[2], E, scale_hi);
 }
 
 __device__ __forceinline__ float point_box_sqdist32(float px, float py, float pz, const float* lo,

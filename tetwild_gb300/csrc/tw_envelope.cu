@@ -595,8 +595,21 @@ __device__ __forceinline__ bool index_point_in(const EnvTree& T, const EpsParams
     return grid_point_in<CERT>(T, E, valid, p, q, st);
 }
 
+// A sorted point as the certified test reads it: its coordinates split in
+// binary32 (p = ph + pl, the split of cert_query) and its index.  One 32-byte
+// sector, written whole by the placing pass and read in order, where a gather
+// of the point's 24 bytes fetches two 64-byte lines of DRAM every other time.
+// 10M points: the test 485 -> 390 us (DRAM reads 840 -> 303 MB for 6M), the
+// placing pass 91 -> 145.
+struct __align__(32) PointRec {
+    float4 a;   // ph0 ph1 ph2 pl0
+    float4 b;   // pl1 pl2 - index
+};
+
 // n_dev (sorted on the dense bin ids): the number of sorted queries, read on
 // the device (the others were decided by the binning pass); else n.
+// rec (DEFER only): the sorted points' records, read in order in place of
+// order and P; nullptr: the point is gathered through order.
 template <int BLOCK, int MINB, bool CERT, bool DEFER>
 __global__ void __launch_bounds__(BLOCK, MINB) k_env_points_bins(const double* __restrict__ P,
                                                            const int32_t* __restrict__ order,
@@ -604,7 +617,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_env_points_bins(const double* _
                                                            uint8_t* __restrict__ out,
                                                            unsigned long long* __restrict__ counters,
                                                            uint32_t* __restrict__ recheck,
-                                                           const uint32_t* __restrict__ n_dev) {
+                                                           const uint32_t* __restrict__ n_dev,
+                                                           const PointRec* __restrict__ rec) {
     TravStats st;
     uint32_t nq = 0;
     if (n_dev) n = min(n, (int64_t)__ldg(n_dev));
@@ -616,9 +630,18 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_env_points_bins(const double* _
         if (i < n) {
             // the points, the order and the answers stream through once
             // (evict-first), so the bins, entries and facet records stay in L2
-            const int64_t j = order ? (int64_t)__ldcs(order + i) : i;
-            const V3 p{__ldcs(P + 3 * j), __ldcs(P + 3 * j + 1), __ldcs(P + 3 * j + 2)};
-            const CertQuery q = cert_query(p, E, T.scale_hi);
+            int64_t j;
+            V3 p;
+            CertQuery q;
+            if (DEFER && rec) {
+                const float4 a = __ldcs(&rec[i].a), b = __ldcs(&rec[i].b);
+                j = (int64_t)__float_as_int(b.w);
+                q = cert_query_split(a.x, a.y, a.z, a.w, b.x, b.y, E, T.scale_hi);
+            } else {
+                j = order ? (int64_t)__ldcs(order + i) : i;
+                p = V3{__ldcs(P + 3 * j), __ldcs(P + 3 * j + 1), __ldcs(P + 3 * j + 2)};
+                q = cert_query(p, E, T.scale_hi);
+            }
             const int r = bins_point_test<CERT, DEFER>(T, E, p, q, st);
             if (DEFER && r == 2) {
                 const uint32_t at = atomicAdd(recheck, 1u);
@@ -1144,6 +1167,22 @@ __global__ void k_point_place(const uint2* __restrict__ bin_rank, int64_t n,
     idx[__ldg(first + br.x) + br.y] = (int32_t)i;
 }
 
+// The same with the points' records in place of their indices.
+__global__ void k_point_place_rec(const double* __restrict__ P,
+                                  const uint2* __restrict__ bin_rank, int64_t n,
+                                  const uint32_t* __restrict__ first, PointRec* __restrict__ rec) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint2 br = __ldcs(bin_rank + i);
+    const V3 p{__ldcs(P + 3 * i), __ldcs(P + 3 * i + 1), __ldcs(P + 3 * i + 2)};
+    if (br.x == 0xffffffffu) return;   // decided by the binning pass
+    float ph[3], pl[3];
+    cert_split(p, ph, pl);
+    PointRec* r = rec + __ldg(first + br.x) + br.y;
+    r->a = make_float4(ph[0], ph[1], ph[2], pl[0]);
+    r->b = make_float4(pl[1], pl[2], 0.0f, __int_as_float((int32_t)i));
+}
+
 // bits a side of the sort grid: the knob (2..8), or the smallest b with
 // 2^(3b) >= n, between 3 and 8 (8: cells of 1/256 of the box, about one
 // envelope-grid cell on a 100k-facet surface)
@@ -1156,7 +1195,8 @@ static int sort_bits(int64_t n, int knob) {
 
 struct SortLayout {
     uint2* bin_rank;
-    int32_t* idx;
+    int32_t* idx;    // sorted point indices, or
+    PointRec* rec;   // records in the same place (nullptr: no room was asked for)
     uint32_t* count;
     int64_t nbins;
     uint32_t* recheck;   // count, then up to n point indices
@@ -1170,13 +1210,15 @@ static size_t cub_scan_bytes(int64_t nbins) {
     return b;
 }
 
-static SortLayout sort_layout(void* base, int64_t n, int knob) {
+static SortLayout sort_layout(void* base, int64_t n, int knob, bool records) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     char* q = static_cast<char*>(base);
     SortLayout L;
     L.nbins = int64_t(1) << (3 * sort_bits(n, knob));
     L.bin_rank = (uint2*)q; q += al(8 * (size_t)n);
-    L.idx = (int32_t*)q; q += al(4 * (size_t)n);
+    L.idx = (int32_t*)q;
+    L.rec = records ? (PointRec*)q : nullptr;
+    q += al((records ? sizeof(PointRec) : 4) * (size_t)n);
     L.count = (uint32_t*)q; q += al(4 * (size_t)L.nbins);
     L.recheck = (uint32_t*)q; q += al(4 * (size_t)n + 4);
     L.temp = q;
@@ -1184,10 +1226,10 @@ static SortLayout sort_layout(void* base, int64_t n, int knob) {
     return L;
 }
 
-size_t env_sort_scratch_bytes(int64_t n, int knob) {
+size_t env_sort_scratch_bytes(int64_t n, int knob, bool records) {
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
     const int64_t nbins = int64_t(1) << (3 * sort_bits(n, knob));
-    return al(8 * (size_t)n) + al(4 * (size_t)n) + al(4 * (size_t)nbins) +
+    return al(8 * (size_t)n) + al((records ? sizeof(PointRec) : 4) * (size_t)n) + al(4 * (size_t)nbins) +
            al(4 * (size_t)n + 4) + al(cub_scan_bytes(nbins)) + 256;
 }
 
@@ -1197,17 +1239,18 @@ constexpr int64_t kSortMin = 4096;
 
 void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2, uint8_t* out,
                        int precision, unsigned long long* counters, void* sort_scratch,
-                       int sort_knob, int point_block, cudaStream_t s, cudaEvent_t ev_begin,
-                       cudaEvent_t ev_end) {
+                       int sort_knob, bool sort_records, int point_block, cudaStream_t s,
+                       cudaEvent_t ev_begin, cudaEvent_t ev_end) {
     if (n <= 0) return;
     const int block = 128;
     const int32_t* order = nullptr;
     uint32_t* recheck = nullptr;
+    PointRec* rec = nullptr;
     const uint32_t* n_dev = nullptr;   // sorted queries, when the binning pass decides some
     const EnvTree T = env_tree_for(S, eps2);
     const EpsParams E = eps_params(eps2);
     if (sort_scratch && n >= kSortMin && n <= INT32_MAX) {
-        SortLayout L = sort_layout(sort_scratch, n, sort_knob);
+        SortLayout L = sort_layout(sort_scratch, n, sort_knob, sort_records);
         const unsigned nb = (unsigned)((n + 255) / 256);
         const int bits = sort_bits(n, sort_knob);
         if (T.boff && T.bid && sort_knob == 1 && (int64_t)T.nocc + 1 <= L.nbins) {
@@ -1241,8 +1284,15 @@ void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2
             size_t tb = L.temp_bytes;
             cub::DeviceScan::ExclusiveSum(L.temp, tb, L.count, (int)L.nbins, s);
         }
-        k_point_place<<<nb, 256, 0, s>>>(L.bin_rank, n, L.count, L.idx);
-        order = L.idx;
+        // the certified bulk test needs no more of a point than its record;
+        // the other tests gather the binary64 coordinates
+        if (L.rec && T.boff && precision == TW_PRECISION_FP32_CERTIFIED) {
+            k_point_place_rec<<<nb, 256, 0, s>>>(P, L.bin_rank, n, L.count, L.rec);
+            rec = L.rec;
+        } else {
+            k_point_place<<<nb, 256, 0, s>>>(L.bin_rank, n, L.count, L.idx);
+            order = L.idx;
+        }
         recheck = L.recheck;
     }
     // the tree-walk kernels: at least 6 blocks of 128 threads per SM (85
@@ -1255,15 +1305,15 @@ void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2
         // for 2 of 512, 0.665 for 1 of 1024)
         cudaMemsetAsync(recheck, 0, 4, s);
         k_env_points_bins<256, 4, true, true><<<grid_for(n, 256, 16), 256, 0, s>>>(
-            P, order, n, T, E, out, counters, recheck, n_dev);
+            P, order, n, T, E, out, counters, recheck, n_dev, rec);
         k_env_points_bins_recheck<<<grid_for(INT32_MAX, 128, 4), 128, 0, s>>>(P, recheck, T, E,
                                                                              out, counters);
     } else if (T.boff && precision == TW_PRECISION_FP32_CERTIFIED) {
         k_env_points_bins<384, 2, true, false><<<grid_for(n, 384, 6), 384, 0, s>>>(
-            P, order, n, T, E, out, counters, nullptr, n_dev);
+            P, order, n, T, E, out, counters, nullptr, n_dev, nullptr);
     } else if (T.boff) {
         k_env_points_bins<384, 2, false, false><<<grid_for(n, 384, 6), 384, 0, s>>>(
-            P, order, n, T, E, out, counters, nullptr, n_dev);
+            P, order, n, T, E, out, counters, nullptr, n_dev, nullptr);
     } else if (T.gslot && precision == TW_PRECISION_FP32_CERTIFIED) {
         // 768 resident threads per SM (85 registers) in every block shape
         switch (point_block) {

@@ -125,8 +125,10 @@ struct Surface {
 // Device scratch for ordering query points by Morton cell before traversal
 // (a counting sort): bin and rank per point, the permutation, the bin counts
 // and the scan temporaries.  knob: the sort_points tuning value (1 = bins
-// sized from n, 2..8 = bits a side).
-size_t env_sort_scratch_bytes(int64_t n, int knob);
+// sized from n, 2..8 = bits a side).  records: room for a 32-byte record per
+// point in place of the permutation (the certified test through the bin index
+// then reads the points in order; without it the points are gathered).
+size_t env_sort_scratch_bytes(int64_t n, int knob, bool records);
 
 // Device memory block owned by a context, grown on demand.
 struct Buffer {
@@ -270,14 +272,14 @@ void free_env_grid(tw_ctx* c, EnvGrid& G);
 // ---- launchers (tw_envelope.cu) ----
 // err: device word; bit 0 = traversal exceeded its bounds, bit 1 = a face
 // exceeded the per-row sample bound.
-// sort_scratch (env_sort_scratch_bytes(n, sort_knob) bytes) enables Morton-ordered
-// traversal; with nullptr the points are traversed in input order.
+// sort_scratch (env_sort_scratch_bytes(n, sort_knob, sort_records) bytes) enables
+// Morton-ordered traversal; with nullptr the points are traversed in input order.
 // precision: TW_PRECISION_FP64 or TW_PRECISION_FP32_CERTIFIED; counters is
 // the context's counter array (error word and statistics).
 void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2, uint8_t* out,
                        int precision, unsigned long long* counters, void* sort_scratch,
-                       int sort_knob, int point_block, cudaStream_t s, cudaEvent_t ev_begin = nullptr,
-                       cudaEvent_t ev_end = nullptr);
+                       int sort_knob, bool sort_records, int point_block, cudaStream_t s,
+                       cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr);
 void launch_env_faces(const Surface& S, const double* tris, int64_t n, double eps2, double sd,
                       uint8_t* out, int precision, unsigned long long* counters, cudaStream_t s);
 void launch_sample_triangle(const double* tri, double sd, double* out, int64_t cap,
