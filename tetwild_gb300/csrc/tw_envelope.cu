@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_env_points_grid(const double* _
 // and the point is in iff one of those leaves tests in (in CERT, the
 // certified binary32 bounds with FP64 in the band; else FP64).
 // ---------------------------------------------------------------------------
-// The point's bin (Morton index) and fine cell (fx + 8 fy + 64 fz).
+// The point's bin (Morton index) and fine cell (fz + 8 fx + 64 fy).
 __device__ __forceinline__ void bin_cell_of(const EnvTree& T, const CertQuery& q, uint32_t& bin,
                                             int& fine) {
     uint32_t m = 0;
@@ -529,7 +529,7 @@ __device__ __forceinline__ void bin_cell_of(const EnvTree& T, const CertQuery& q
             f = min((int)(__fsub_rn(t, (float)i) * (float)kFine), kFine - 1);
         }
         m |= morton_expand10((uint32_t)i) << (2 - k);
-        fine += f * (k == 0 ? 1 : (k == 1 ? kFine : kFine * kFine));
+        fine += f * (k == 2 ? 1 : (k == 0 ? kFine : kFine * kFine));
     }
     bin = m;
 }
@@ -728,9 +728,16 @@ static SatGrid sat_grid(const float* lo, const int64_t* n, double inv_c, double 
 struct SatSlab {
     float a[3];
     float lo, hi;
-    float inv;   // 1 / (a[2] cs), 0: the axis does not depend on z
 };
 constexpr int kSlabs = 13;
+
+// A slab in units of cells along z: the cell with centre (wx, wy, wz + cs i)
+// is within it when l - q <= i <= h - q, q = ax wx + ay wy + az wz.  dq: q's
+// step to the column four cells on in y.
+struct __align__(32) ColumnSlab {
+    float ax, ay, az, l;
+    float h, dq, pad[2];
+};
 
 // One lane's leaf: vertices relative to t0, the grid's origin relative to t0,
 // the error scale and the index box of the leaf grown by Rm.
@@ -745,6 +752,7 @@ constexpr int kSatWarps = kSatBlock / 32;
 struct SatShared {
     SatLeaf leaf[kSatWarps][32];
     SatSlab slab[kSatWarps][kSlabs + 3];
+    ColumnSlab column[kSatWarps][kSlabs];
 };
 
 // false when the box spans more than limit cells
@@ -779,7 +787,7 @@ __device__ __forceinline__ bool sat_prepare(const double* __restrict__ tri, int6
 }
 
 // The leaf's slabs (the whole warp); half: the tested cube's half-size.
-__device__ __forceinline__ void sat_slabs(const SatLeaf& l, float half, float cs, SatSlab* slab) {
+__device__ __forceinline__ void sat_slabs(const SatLeaf& l, float half, SatSlab* slab) {
     const int j = threadIdx.x & 31;
     __syncwarp();
     if (j < kSlabs) {
@@ -823,8 +831,6 @@ __device__ __forceinline__ void sat_slabs(const SatLeaf& l, float half, float cs
         s.a[2] = a[2];
         s.lo = use ? fminf(0.0f, fminf(p1, p2)) - r : -inf;
         s.hi = use ? fmaxf(0.0f, fmaxf(p1, p2)) + r : inf;
-        const float dz = a[2] * cs;
-        s.inv = fabsf(dz) > 1e-32f ? 1.0f / dz : 0.0f;
     }
     __syncwarp();
 }
@@ -875,7 +881,7 @@ __device__ __forceinline__ void sat_cells(const double* __restrict__ tri, int32_
     for (unsigned left = __ballot_sync(0xffffffffu, ok); left; left &= left - 1) {
         const int k = __ffs(left) - 1;
         const SatLeaf& l = sh.leaf[warp][k];
-        sat_slabs(l, g.hf, g.csf, sh.slab[warp]);
+        sat_slabs(l, g.hf, sh.slab[warp]);
         const int nbox = l.nb[0] * l.nb[1] * l.nb[2];
         uint32_t at = fcnt ? 0u : __ldg(foff + f0 + k);
         const uint32_t end = fcnt ? 0xffffffffu : __ldg(foff + f0 + k + 1);
@@ -944,66 +950,92 @@ __device__ __forceinline__ uint32_t morton_compact10(uint32_t v) {
     return v;
 }
 
-// The fine-cell mask of every entry: bit fx + 8 fy + 64 fz set when the
-// bin's fine cell (a grid of 8n cells a side: g) is within reach of the leaf.
-// A lane takes two columns of eight cells along z (fx, fy = lane % 8, lane / 8
-// and lane / 8 + 4); each slab leaves an interval of a column, so a column
-// costs its 13 slabs once instead of a 13-axis test per cell (100k facets:
-// 13.1 ms in two passes, counting and filling; 1.3 ms here, the count taking
-// whole bins), and the ballots of cell fz of the first and second columns are
-// the mask's words 2 fz and 2 fz + 1.  The
-// quotients below are off by 2^-22 of |a|_1 L in the projection, far inside
-// the margin.
+// The slabs in units of cells along z (the whole warp).  An axis with |a_z| <
+// 2^-20 |a|_1 takes 2^-20 |a|_1 for a_z in the unit: its projection moves by
+// at most 7 of those units over a column, so its interval, 8 wider below and
+// 16 above, holds all of a column that a cell of it is within.  An axis whose
+// numbers could leave binary32 is not used.
+__device__ __forceinline__ void column_slabs(const SatLeaf& l, const SatSlab* slab, float cs,
+                                             ColumnSlab* column) {
+    const int j = threadIdx.x & 31;
+    if (j < kSlabs) {
+        const float a0 = slab[j].a[0], a1 = slab[j].a[1], a2 = slab[j].a[2];
+        const float n1 = fabsf(a0) + fabsf(a1) + fabsf(a2);
+        const bool flat = !(fabsf(a2) >= n1 * 0x1p-20f);
+        const float inv = flat ? 0x1p20f / (n1 * cs) : 1.0f / (a2 * cs);
+        const bool use = n1 >= 0x1p-40f && fabsf(inv) * n1 * l.mL < 0x1p80f;   // false for NaN
+        const float inf = __int_as_float(0x7f800000);
+        const float u = slab[j].lo * inv, v = slab[j].hi * inv;
+        ColumnSlab c;
+        c.ax = use ? a0 * inv : 0.0f;
+        c.ay = use ? a1 * inv : 0.0f;
+        c.az = use ? a2 * inv : 0.0f;
+        c.l = use ? fminf(u, v) - (flat ? 8.0f : 0.0f) : -inf;
+        c.h = use ? fmaxf(u, v) + (flat ? 16.0f : 0.0f) : inf;
+        c.dq = c.ay * (4.0f * cs);
+        column[j] = c;
+    }
+    __syncwarp();
+}
+
+// The fine-cell mask of every entry, 16 words an entry: bit fz + 8 fx + 64 fy
+// set when the bin's fine cell (a grid of 8n cells a side: g) is within reach
+// of the leaf.  A lane takes two columns of eight cells along z (fx, fy =
+// lane % 8, lane / 8 and lane / 8 + 4); each slab leaves an interval of a
+// column, which is a byte of the mask, and four lanes make two words.  Bound
+// by its instructions, so a column costs its 13 slabs once instead of a
+// 13-axis test per cell (100k facets: 13.1 ms in two passes, counting and
+// filling; 1.28 ms, the count taking whole bins), the slabs are scaled once a leaf
+// (four differences and bounds a slab and two columns where a quotient took
+// twice that) and the mask's bits lie along the columns (ballots of the cells
+// across them took 80 instructions more): 0.62 ms.  The scaled numbers are off by
+// 10 2^-24 |a|_1 L in the projection, inside the margin.
 __global__ void __launch_bounds__(kSatBlock) k_bin_masks(const double* __restrict__ tri, int32_t nf,
                                                          SatGrid g, const uint32_t* __restrict__ foff,
                                                          const uint32_t* __restrict__ keys,
-                                                         uint32_t* __restrict__ masks, int64_t ntot) {
+                                                         uint32_t* __restrict__ masks) {
     __shared__ SatShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t f0 = ((int64_t)blockIdx.x * kSatWarps + warp) * 32;
     if (f0 >= nf) return;   // whole warps
     if (f0 + lane < nf) sat_prepare(tri, f0 + lane, g, INT64_MAX, sh.leaf[warp][lane]);
     const int leaves = (int)(nf - f0 < 32 ? nf - f0 : 32);
-    const SatSlab* slab = sh.slab[warp];
+    const ColumnSlab* column = sh.column[warp];
     for (int k = 0; k < leaves; ++k) {
         const SatLeaf& l = sh.leaf[warp][k];
-        sat_slabs(l, g.hf, g.csf, sh.slab[warp]);
+        sat_slabs(l, g.hf, sh.slab[warp]);
+        column_slabs(l, sh.slab[warp], g.csf, sh.column[warp]);
         const uint32_t end = __ldg(foff + f0 + k + 1);
         for (uint32_t at = __ldg(foff + f0 + k); at < end; ++at) {
             const uint32_t key = __ldg(keys + at);
             const float x = (float)(kFine * morton_compact10(key >> 2) + (lane & 7));
             const float y = (float)(kFine * morton_compact10(key >> 1) + (lane >> 3));
             const float z = (float)(kFine * morton_compact10(key));
-            const float wx = l.base[0] + (x + 0.5f) * g.csf, wz = l.base[2] + (z + 0.5f) * g.csf;
-            const float wy0 = l.base[1] + (y + 0.5f) * g.csf;
-            const float wy1 = l.base[1] + (y + 4.5f) * g.csf;
+            const float wx = l.base[0] + (x + 0.5f) * g.csf, wy = l.base[1] + (y + 0.5f) * g.csf,
+                        wz = l.base[2] + (z + 0.5f) * g.csf;
             float l0 = 0.0f, h0 = 7.0f, l1 = 0.0f, h1 = 7.0f;
 #pragma unroll
             for (int j = 0; j < kSlabs; ++j) {
-                const float t = slab[j].a[0] * wx + slab[j].a[2] * wz;
-                const float t0 = t + slab[j].a[1] * wy0, t1 = t + slab[j].a[1] * wy1;
-                const float lo = slab[j].lo, hi = slab[j].hi, inv = slab[j].inv;
-                if (inv == 0.0f) {   // the same on every lane
-                    if (t0 < lo || t0 > hi) h0 = -1.0f;
-                    if (t1 < lo || t1 > hi) h1 = -1.0f;
-                } else {
-                    const float u0 = (lo - t0) * inv, v0 = (hi - t0) * inv;
-                    const float u1 = (lo - t1) * inv, v1 = (hi - t1) * inv;
-                    l0 = fmaxf(l0, fminf(u0, v0));
-                    h0 = fminf(h0, fmaxf(u0, v0));
-                    l1 = fmaxf(l1, fminf(u1, v1));
-                    h1 = fminf(h1, fmaxf(u1, v1));
-                }
+                const ColumnSlab& c = column[j];
+                const float q0 = fmaf(c.ax, wx, fmaf(c.ay, wy, c.az * wz)), q1 = q0 + c.dq;
+                l0 = fmaxf(l0, c.l - q0);
+                h0 = fminf(h0, c.h - q0);
+                l1 = fmaxf(l1, c.l - q1);
+                h1 = fminf(h1, c.h - q1);
             }
-            uint32_t mine = 0;
-#pragma unroll
-            for (int fz = 0; fz < kFine; ++fz) {
-                const unsigned b0 = __ballot_sync(0xffffffffu, l0 <= (float)fz && (float)fz <= h0);
-                const unsigned b1 = __ballot_sync(0xffffffffu, l1 <= (float)fz && (float)fz <= h1);
-                if (lane == 2 * fz) mine = b0;
-                if (lane == 2 * fz + 1) mine = b1;
-            }
-            if (lane < kFineWords) masks[(int64_t)lane * ntot + at] = mine;
+            // the cells ceil(l) .. floor(h) of each column, none for l > 7 or h < 0
+            const int i0 = (int)ceilf(fminf(l0, 8.0f)), i1 = (int)ceilf(fminf(l1, 8.0f));
+            const int e0 = (int)floorf(fmaxf(h0, -1.0f)), e1 = (int)floorf(fmaxf(h1, -1.0f));
+            const uint32_t m0 = (0xffu >> (7 - e0)) & (0xffu << i0);
+            const uint32_t m1 = (0xffu >> (7 - e1)) & (0xffu << i1);
+            const int sh8 = 8 * (lane & 3);
+            uint32_t w0 = (m0 & 0xffu) << sh8, w1 = (m1 & 0xffu) << sh8;
+            w0 |= __shfl_xor_sync(0xffffffffu, w0, 1);
+            w1 |= __shfl_xor_sync(0xffffffffu, w1, 1);
+            w0 |= __shfl_xor_sync(0xffffffffu, w0, 2);
+            w1 |= __shfl_xor_sync(0xffffffffu, w1, 2);
+            if ((lane & 3) < 2)
+                masks[(int64_t)at * kFineWords + (lane >> 2) + 8 * (lane & 3)] = lane & 1 ? w1 : w0;
         }
     }
 }
@@ -1017,8 +1049,15 @@ __global__ void k_bin_split(const uint32_t* __restrict__ keys, const uint32_t* _
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int64_t from = src[i];
+    const uint4* m = reinterpret_cast<const uint4*>(masks + from * kFineWords);
 #pragma unroll
-    for (int w = 0; w < kFineWords; ++w) ent[w * n + i] = masks[w * n + from];
+    for (int w = 0; w < kFineWords / 4; ++w) {
+        const uint4 v = __ldg(m + w);
+        ent[(4 * w) * n + i] = v.x;
+        ent[(4 * w + 1) * n + i] = v.y;
+        ent[(4 * w + 2) * n + i] = v.z;
+        ent[(4 * w + 3) * n + i] = v.w;
+    }
     ent[kFineWords * n + i] = leaves[from];
     atomicAdd(cnt + keys[i], 1u);
 }
@@ -2584,7 +2623,7 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
                  *leaves = (uint32_t*)(w + o_lf), *masks = (uint32_t*)(w + o_m),
                  *bcnt = (uint32_t*)(w + o_bc);
         k_bin_cells<<<leaf_grid, kSatBlock, 0, s>>>(S.tri, nf, GB, bfoff, keys, vals, leaves);
-        k_bin_masks<<<leaf_grid, kSatBlock, 0, s>>>(S.tri, nf, GF, bfoff, keys, masks, bt);
+        k_bin_masks<<<leaf_grid, kSatBlock, 0, s>>>(S.tri, nf, GF, bfoff, keys, masks);
         t1 = tb;
         cub::DeviceRadixSort::SortPairs(temp, t1, keys, keys2, vals, vals2, (int)bt, 0,
                                         std::max(1, 3 * bits), s);
