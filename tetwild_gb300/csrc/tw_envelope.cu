@@ -725,9 +725,9 @@ static SatGrid sat_grid(const float* lo, const int64_t* n, double inv_c, double 
 // 8 2^-24 |a|_1 L, so each is within |a|_1 2^-19 L (1 + 2^-1); an axis
 // separates only by more than |a|_1 2^-18 L.  Cells no axis separates by that
 // margin are kept (a longer list, never a missing leaf).
-struct SatSlab {
+struct __align__(32) SatSlab {
     float a[3];
-    float lo, hi;
+    float lo, hi, pad[3];
 };
 constexpr int kSlabs = 13;
 
@@ -840,7 +840,7 @@ __device__ __forceinline__ bool sat_within(const SatSlab* slab, float wx, float 
     bool in = true;
 #pragma unroll
     for (int j = 0; j < kSlabs; ++j) {
-        const float p = slab[j].a[0] * wx + slab[j].a[1] * wy + slab[j].a[2] * wz;
+        const float p = fmaf(slab[j].a[0], wx, fmaf(slab[j].a[1], wy, slab[j].a[2] * wz));
         in = in && !(p < slab[j].lo) && !(p > slab[j].hi);
     }
     return in;
