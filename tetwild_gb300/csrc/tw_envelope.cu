@@ -745,12 +745,16 @@ struct SatLeaf {
     float v1[3], v2[3], base[3], mL;
     int32_t i0[3], nb[3];
 };
-// Each warp prepares 32 leaves, one a lane (their binary64 work would cost a
-// warp per leaf 32 times as much), and then takes them in turn.
+// A block's first warp prepares 32 leaves, one a lane (their binary64 work
+// would cost a warp per leaf 32 times as much), and then the warps take them in
+// turn.  With 32 leaves a warp, 3k warps in all, the leaves with the most cells
+// held the launch: a quarter of the warps resident on the average (100k
+// facets: counts 0.22 ms, grid cells 0.14, bin cells 0.091; now 0.155, 0.097,
+// 0.071).
 constexpr int kSatBlock = 128;
 constexpr int kSatWarps = kSatBlock / 32;
 struct SatShared {
-    SatLeaf leaf[kSatWarps][32];
+    SatLeaf leaf[32];
     SatSlab slab[kSatWarps][kSlabs + 3];
     ColumnSlab column[kSatWarps][kSlabs];
 };
@@ -867,20 +871,24 @@ __device__ __forceinline__ void sat_cells(const double* __restrict__ tri, int32_
                                           const uint32_t* __restrict__ foff,
                                           int* __restrict__ too_big, Fill fill) {
     __shared__ SatShared sh;
+    __shared__ unsigned usable;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t f0 = ((int64_t)blockIdx.x * kSatWarps + warp) * 32;
-    if (f0 >= nf) return;   // whole warps
-    const bool have = f0 + lane < nf;
-    bool ok = false;
-    if (have) {
-        ok = sat_prepare(tri, f0 + lane, g, limit, sh.leaf[warp][lane]);
-        if (!ok && too_big) atomicExch(too_big, 1);
+    const int64_t f0 = (int64_t)blockIdx.x * 32;
+    if (warp == 0) {
+        bool ok = false;
+        if (f0 + lane < nf) {
+            ok = sat_prepare(tri, f0 + lane, g, limit, sh.leaf[lane]);
+            if (!ok && too_big) atomicExch(too_big, 1);
+            if (!ok && fcnt) fcnt[f0 + lane] = 0;
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, ok);
+        if (lane == 0) usable = b;
     }
-    uint32_t mine = 0;
+    __syncthreads();
     unsigned long long sum = 0;
-    for (unsigned left = __ballot_sync(0xffffffffu, ok); left; left &= left - 1) {
-        const int k = __ffs(left) - 1;
-        const SatLeaf& l = sh.leaf[warp][k];
+    for (int k = warp; k < 32; k += kSatWarps) {
+        if (!((usable >> k) & 1u)) continue;
+        const SatLeaf& l = sh.leaf[k];
         sat_slabs(l, g.hf, sh.slab[warp]);
         const int nbox = l.nb[0] * l.nb[1] * l.nb[2];
         uint32_t at = fcnt ? 0u : __ldg(foff + f0 + k);
@@ -893,13 +901,10 @@ __device__ __forceinline__ void sat_cells(const double* __restrict__ tri, int32_
             if (!fcnt && in && w < end) fill(w, (int32_t)(f0 + k), x, y, z);
             at += __popc(bal);
         }
-        if (lane == k) mine = at;
+        if (fcnt && lane == 0) fcnt[f0 + k] = at;
         sum += at;
     }
-    if (fcnt) {
-        if (have) fcnt[f0 + lane] = mine;
-        if (lane == 0 && sum) atomicAdd(total, sum);
-    }
+    if (fcnt && lane == 0 && sum) atomicAdd(total, sum);
 }
 constexpr int64_t kMaxLeafCells = 65536, kMaxLeafBins = 4096;
 
@@ -988,7 +993,8 @@ __device__ __forceinline__ void column_slabs(const SatLeaf& l, const SatSlab* sl
 // filling; 1.28 ms, the count taking whole bins), the slabs are scaled once a leaf
 // (four differences and bounds a slab and two columns where a quotient took
 // twice that) and the mask's bits lie along the columns (ballots of the cells
-// across them took 80 instructions more): 0.62 ms.  The scaled numbers are off by
+// across them took 80 instructions more): 0.62 ms, and
+// 0.46 with a block's warps sharing its 32 leaves.  The scaled numbers are off by
 // 10 2^-24 |a|_1 L in the projection, inside the margin.
 __global__ void __launch_bounds__(kSatBlock) k_bin_masks(const double* __restrict__ tri, int32_t nf,
                                                          SatGrid g, const uint32_t* __restrict__ foff,
@@ -996,13 +1002,13 @@ __global__ void __launch_bounds__(kSatBlock) k_bin_masks(const double* __restric
                                                          uint32_t* __restrict__ masks) {
     __shared__ SatShared sh;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t f0 = ((int64_t)blockIdx.x * kSatWarps + warp) * 32;
-    if (f0 >= nf) return;   // whole warps
-    if (f0 + lane < nf) sat_prepare(tri, f0 + lane, g, INT64_MAX, sh.leaf[warp][lane]);
+    const int64_t f0 = (int64_t)blockIdx.x * 32;
+    if (warp == 0 && f0 + lane < nf) sat_prepare(tri, f0 + lane, g, INT64_MAX, sh.leaf[lane]);
+    __syncthreads();
     const int leaves = (int)(nf - f0 < 32 ? nf - f0 : 32);
     const ColumnSlab* column = sh.column[warp];
-    for (int k = 0; k < leaves; ++k) {
-        const SatLeaf& l = sh.leaf[warp][k];
+    for (int k = warp; k < leaves; k += kSatWarps) {
+        const SatLeaf& l = sh.leaf[k];
         sat_slabs(l, g.hf, sh.slab[warp]);
         column_slabs(l, sh.slab[warp], g.csf, sh.column[warp]);
         const uint32_t end = __ldg(foff + f0 + k + 1);
@@ -2511,7 +2517,7 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     unsigned long long* acc = (unsigned long long*)(q + o_acc);
     uint32_t *fcnt = (uint32_t*)(q + o_cnt), *foff = (uint32_t*)(q + o_off);
     uint32_t *bfcnt = (uint32_t*)(q + o_bcnt), *bfoff = (uint32_t*)(q + o_boff);
-    const unsigned leaf_grid = (unsigned)(((int64_t)nf + kSatBlock - 1) / kSatBlock);
+    const unsigned leaf_grid = (unsigned)(((int64_t)nf + 31) / 32);   // 32 leaves a block
     cudaMemsetAsync(acc, 0, 64, s);
     cudaMemsetAsync(fcnt + nf, 0, 4, s);
     cudaMemsetAsync(bfcnt + nf, 0, 4, s);
