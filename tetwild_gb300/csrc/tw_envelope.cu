@@ -9,11 +9,12 @@
 // facet that tests <= eps2 is ever skipped, so the decision equals the
 // brute-force decision over all facets.
 //
-// Faces (isFaceOutEnvelop_sampling, :1046-1109): a warp per face; the lanes
-// generate sampleTriangle's samples (Common.cpp:143-228) with the same
-// arithmetic as the reference order, each lane first retests the facet that
-// held its previous sample (the reference's prev_facet hint, :1080-1083),
-// and the warp stops at the first sample that is out.
+// Faces (isFaceOutEnvelop_sampling, :1046-1109): first the pieces of a face
+// that lie inside as a whole (tw_hull.cuh); where pieces stay open, a warp
+// generates sampleTriangle's samples there (Common.cpp:143-228) with the same
+// arithmetic as the reference order, tests them, the facet that held the
+// previous samples first (the reference's prev_facet hint, :1080-1083), and
+// stops at the first sample that is out.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_run_length_encode.cuh>
 #include <cub/device/device_scan.cuh>
@@ -1346,8 +1347,9 @@ void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2
     if (ev_begin) cudaEventRecord(ev_begin, s);
     if (T.boff && precision == TW_PRECISION_FP32_CERTIFIED && recheck) {
         // no FP64 code in the bulk kernel (64 registers): 4 blocks of 256 per SM
-        // (measured on 10M points: 0.564 ms against 0.592 for 8 of 128, 0.646
-        // for 2 of 512, 0.665 for 1 of 1024)
+        // (10M points, gathered: 0.564 ms against 0.592 for 8 of 128, 0.646 for 2
+        // of 512, 0.665 for 1 of 1024; from records: 0.39 against 0.49, 0.56 and
+        // 0.72 for 5, 6 and 8 blocks of 256)
         cudaMemsetAsync(recheck, 0, 4, s);
         k_env_points_bins<256, 4, true, true><<<grid_for(n, 256, 16), 256, 0, s>>>(
             P, order, n, T, E, out, counters, recheck, n_dev, rec);
@@ -1860,7 +1862,7 @@ __device__ __forceinline__ int face_prepare(const double* t, double sd, bool sha
 // of the sampling's 128 registers, and half of its stalls were barriers.)
 // Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
 // to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
-// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.2 and 0.27.
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 1.98 and 0.25.
 // Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
 constexpr int kFaceWarps = kFaceBlock / 32;
