@@ -1862,7 +1862,7 @@ __device__ __forceinline__ int face_prepare(const double* t, double sd, bool sha
 // of the sampling's 128 registers, and half of its stalls were barriers.)
 // Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
 // to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
-// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 1.98 and 0.25.
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.1 and 0.25.
 // Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
 constexpr int kFaceWarps = kFaceBlock / 32;
