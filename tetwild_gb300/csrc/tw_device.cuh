@@ -550,14 +550,13 @@ static __device__ __noinline__ double rf_tiny(const double* T) {
                   (kRfTiny * ((x0 + hx) - 3.0 * x3)) * x3);
 }
 // fl(a - fl(tiny z)) for tiny = tf to 3e-7: a correction of a few units.  z is
-// zero or at least 2^-126: a smaller one has no binary32 value, and beside
-// coordinates of 1e5 and more its correction still reaches a's last places
-// (an underflow of tf z costs at most 2^-23 units).
+// at least 2^-126 (a smaller one has no binary32 value, and beside coordinates
+// of 1e5 and more its correction still reaches a's last places; an underflow of
+// tf z costs at most 2^-23 units), or zero or subnormal, far below any unit.
 __device__ __forceinline__ double sub_tiny(double a, float tf, double z, bool ok,
                                            const double* T) {
     const int ea = exponent_field(a), ez = exponent_field(z);
-    const bool zero = (((uint32_t)__double2hiint(z) << 1) | (uint32_t)__double2loint(z)) == 0u;
-    ok = ok && ea > 948 && ea < 1200 && ez < 1100 && (ez >= 897 || zero);
+    ok = ok && ea > 948 && ea < 1200 && ez < 1100 && (ez >= 897 || ez == 0);
     const float zs = ez < 897 ? 0.0f : significand32(z) * __uint_as_float((uint32_t)(ez - 896) << 23);
     const uint32_t sgn = ((uint32_t)__double2hiint(a) ^ (uint32_t)__double2hiint(z)) & 0x80000000u;
     const float mag = tf * zs * __uint_as_float((uint32_t)(1202 - max(948, min(ea, 1200))) << 23);
@@ -659,7 +658,7 @@ __device__ __forceinline__ void amips_rf_hessian_in(const double* T, int ce, dou
     H[2] = rneg * (un * v3 + a2);
     H[3] = rneg * (a1 + w1 * v2);
     H[4] = r * ((((-(s * s)) * k49n + (s * k43) * ly) + (s * nd) * v1) + 3.0);
-    H[5] = rneg * (sub_tiny(-(v3 * w1), tf, x1, tok, T) + a3);
+    H[5] = rneg * (a3 - sub_tiny(v3 * w1, tf, -x1, tok, T));   // (a zero may have the other sign)
     H[6] = rneg * (sub_tiny(a2, tf, y1, tok, T) + w2 * v2);
     H[7] = rneg * (a3 - w2 * v1);
     H[8] = r * ((((-lz) * t) * k43 - (kRf10_9 * (t * t)) * nd) + 3.0);
