@@ -879,6 +879,9 @@ __device__ __forceinline__ int orient3d_staged(const double* p, const double* q,
 // Orientation sign of det[d1, d2, d3] when binary32 can certify it, else 2.
 // The bound adds the rounding of the FP64 differences (3.01 u per term of the
 // permanent) to the stage-A bound (7 + 56 u) u of the binary32 evaluation.
+// What underflows (differences, their products) is off by 2^-150 each: with m2
+// the sum of their squares, 18 m2 + 6 sqrt(m2) + 3 of those in all, which the
+// 0.98 u left of the bound cover when the permanent is above 1e-30 + 2^-120 m2.
 __device__ __forceinline__ int orient32_filter(const float* d1, const float* d2, const float* d3) {
     float vywz = d2[1] * d3[2], vzwy = d2[2] * d3[1];
     float vzwx = d2[2] * d3[0], vxwz = d2[0] * d3[2];
@@ -887,7 +890,10 @@ __device__ __forceinline__ int orient32_filter(const float* d1, const float* d2,
     float perm = (fabsf(d1[0]) * (fabsf(vywz) + fabsf(vzwy)) +
                   fabsf(d1[1]) * (fabsf(vzwx) + fabsf(vxwz))) +
                  fabsf(d1[2]) * (fabsf(vxwy) + fabsf(vywx));
-    if (!(perm > 1e-30f) || !(perm < 1e30f)) return 2;
+    float m2 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m2 = fmaf(d1[k], d1[k], fmaf(d2[k], d2[k], fmaf(d3[k], d3[k], m2)));
+    if (!(perm > fmaf(m2, 0x1p-120f, 1e-30f)) || !(perm < 1e30f)) return 2;
     float bound = 11.0f * kU32 * perm;
     if (det > bound) return 1;
     if (-det > bound) return -1;
