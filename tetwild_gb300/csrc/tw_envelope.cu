@@ -2351,9 +2351,10 @@ __device__ __forceinline__ bool nearest_facet_grid(const EnvTree& T, double eps2
             umin = fminf(umin, U2);
         }
     }
-    // slack = 16 u64 M = Mu2 / 32 (Mu2 = 16 u^2 M, u64 = u^2 / 32)
+    // slack = 16 u64 M = Mu2 / 32 (Mu2 = 16 u^2 M, u64 = u^2 / 32); from 1e-35 on
+    // what a bound's squares lose to underflow, below 2^-147, is far inside the 2^-18
     const float t = __fmul_ru(__fadd_ru(__fsqrt_ru(umin), cq.Mu2), 1.00000381f);
-    const float lim = __fmul_ru(t, t);
+    const float lim = fmaxf(__fmul_ru(t, t), 1e-35f);
     double best = INFINITY;
     int32_t best_id = 0x7fffffff;
     V3 best_q{0.0, 0.0, 0.0};
