@@ -219,6 +219,14 @@ struct Guard {
 
 // scratch slot layout: pipelines use slots [0, kNumPipe), their point-ordering
 // scratch [3, 3 + kNumPipe), misc uses 6, 7
+
+// Queues the clearing of n counters on the context's stream.  Not cudaMemset:
+// it runs on the legacy default stream, which the context's streams (made
+// non-blocking) are not ordered against, and does not wait for the device.
+cudaError_t clear_counters(tw_ctx* c, int first, int n) {
+    return cudaMemsetAsync(c->counters + first, 0, (size_t)n * sizeof(unsigned long long), c->stream);
+}
+
 // Waits for the context's streams.  The error word comes back by a copy queued
 // behind the work, so one wait serves both (a blocking copy after three waits
 // cost a 37-point call 12 of its 48 us); the pipeline's other streams are
@@ -240,7 +248,8 @@ int sync_status(tw_ctx* c, const char* where) {
     // device-side error word: read and clear
     const unsigned long long err = c->host_words[0];
     if (err) {
-        cudaMemset(c->counters + kCntError, 0, sizeof(err));
+        // cleared before the call returns: the next one may start on another stream
+        if (clear_counters(c, kCntError, 1) == cudaSuccess) cudaStreamSynchronize(c->stream);
         std::string m = std::string(where) + ": ";
         if (err & 1ULL) m += "surface traversal exceeded its bounds (corrupt tree); ";
         if (err & 2ULL) m += "a face exceeds the per-row sample bound (4e6 samples); ";
@@ -337,7 +346,12 @@ int tw_ctx_create(int device, size_t hbm_budget_bytes, tw_ctx** out) {
         return TW_ERR_OOM;
     }
     c->host_words = (unsigned long long*)words;
-    cudaMemset(c->counters, 0, kNumCounters * sizeof(unsigned long long));
+    if (clear_counters(c, 0, kNumCounters) != cudaSuccess ||
+        cudaStreamSynchronize(c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        tw_ctx_destroy(c);
+        return TW_ERR_CUDA;
+    }
     *out = c;
     return TW_OK;
 }
@@ -506,8 +520,8 @@ int tw_reset_stats(tw_ctx* c) {
     if (st != TW_OK) return st;
     const int keep[] = {kCntExactOrient, kCntEnvQueries, kCntEnvFacetTests, kCntEnvFp64,
                         kCntAmipsTets, kCntAmipsFp64, kCntEnvWarpFallback};
-    for (int k : keep) cudaMemset(c->counters + k, 0, sizeof(unsigned long long));
-    return sync_status(c, "tw_reset_stats");
+    for (int k : keep) clear_counters(c, k, 1);
+    return sync_status(c, "tw_reset_stats");   // waits for them
 }
 
 // ---- AMIPS -------------------------------------------------------------------
