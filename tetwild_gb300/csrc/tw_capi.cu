@@ -47,6 +47,12 @@ void dev_free(tw_ctx* c, void* p, size_t bytes) {
     c->used -= std::min(c->used, bytes);
 }
 
+// scratch slot layout: pipelines use slots [0, kNumPipe), their point-ordering
+// scratch [kSortSlots, kSortSlots + kNumPipe) and records [kRecordSlots,
+// kRecordSlots + kNumPipe), the other calls 6 to 9
+constexpr int kNumPipe = 3, kSortSlots = 3, kRecordSlots = 10;
+static_assert(sizeof(tw_ctx::scratch) / sizeof(Buffer) == kRecordSlots + kNumPipe, "scratch slots");
+
 int ensure(tw_ctx* c, int slot, size_t bytes, void** out) {
     Buffer& b = c->scratch[slot];
     if (b.cap < bytes) {
@@ -62,17 +68,42 @@ int ensure(tw_ctx* c, int slot, size_t bytes, void** out) {
     return TW_OK;
 }
 
-// Scratch for sorting n points: with room for the points' records (records set)
-// up to 128M points (32 bytes each), and without it above that, in a context
-// that is held to a memory budget, and where the device has no room for them.
-int ensure_sort(tw_ctx* c, int slot, int64_t n, void** out, bool* records) {
-    *records = n <= (int64_t(1) << 27) && !c->budget;
-    if (*records) {
-        if (ensure(c, slot, env_sort_scratch_bytes(n, c->sort_points, true), out) == TW_OK)
-            return TW_OK;
-        *records = false;
+// Scratch of a point batch: *out for sorting n points, with room for their
+// records (*records == *out) where the test reads them.  A buffer that serves
+// without records stays as it is (work captured with it may be replayed), and
+// the records get one of their own (slot kRecordSlots on).  nullptr: no records,
+// so above 128M points, in a context that is held to a memory budget, where the
+// device had no room for as much before (records_refused: not asked for again
+// until a surface is uploaded), and in a stream capture that would have to
+// allocate them.
+int ensure_sort(tw_ctx* c, int slot, const Surface& S, int64_t n, void** out, void** records) {
+    const size_t plain = env_sort_scratch_bytes(n, c->sort_points, false);
+    *records = nullptr;
+    if (n <= (int64_t(1) << 27) && !c->budget &&
+        env_points_use_records(S, n, c->eps2, c->precision, c->sort_points)) {
+        const size_t with = env_sort_scratch_bytes(n, c->sort_points, true);
+        const size_t held = c->scratch[slot].cap;
+        const bool apart = held >= plain && held < with;
+        const int at = apart ? kRecordSlots + slot - kSortSlots : slot;
+        const size_t bytes = apart ? env_record_bytes(n) : with;
+        bool ask = true;
+        if (bytes > c->scratch[at].cap) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            cudaStreamIsCapturing(c->stream, &cap);
+            ask = bytes < c->records_refused && cap == cudaStreamCaptureStatusNone;
+        }
+        if (ask) {
+            const std::string said = c->last_error;
+            if (ensure(c, at, bytes, records) == TW_OK) {
+                *out = apart ? c->scratch[slot].ptr : *records;
+                return TW_OK;
+            }
+            c->last_error = said;   // no error of the call: it goes on without records
+            c->records_refused = bytes;
+            *records = nullptr;
+        }
     }
-    return ensure(c, slot, env_sort_scratch_bytes(n, c->sort_points, false), out);
+    return ensure(c, slot, plain, out);
 }
 
 // ---- pipe peak probes -------------------------------------------------------
@@ -208,7 +239,6 @@ static double __longlong_as_double_host(unsigned long long b) {
 
 namespace {
 
-constexpr int kNumPipe = 3;
 // point chunks of the host-buffer envelope call: the copy of one chunk
 // overlaps the test of the one before, and the last chunk's test is the tail
 constexpr size_t kPointChunkBytes = 96ull << 20;
@@ -217,8 +247,6 @@ struct Guard {
     explicit Guard(int dev) { cudaSetDevice(dev); }
 };
 
-// scratch slot layout: pipelines use slots [0, kNumPipe), their point-ordering
-// scratch [3, 3 + kNumPipe), misc uses 6, 7
 
 // Queues the clearing of n counters on the context's stream.  Not cudaMemset:
 // it runs on the legacy default stream, which the context's streams (made
@@ -756,6 +784,7 @@ int tw_surface_upload(tw_ctx* c, const double* V, int32_t nv, const int32_t* F, 
     }
     cudaMemcpyAsync(dV, V, 24 * (size_t)nv, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(dF, F, 12 * (size_t)nf, cudaMemcpyHostToDevice, c->stream);
+    c->records_refused = SIZE_MAX;
     st = build_surface(c, c->surf[which], (const double*)dV, nv, (const int32_t*)dF, nf, c->stream);
     dev_free(c, dV, 24 * (size_t)nv);
     dev_free(c, dF, 12 * (size_t)nf);
@@ -769,8 +798,8 @@ int tw_envelope_points_device(tw_ctx* c, const double* P, int64_t n, int which, 
     if (c->surf[which].nf == 0) return fail(c, TW_ERR_NO_SURFACE, "no surface uploaded");
     Guard g(c->device);
     void* sort = nullptr;
-    bool records;
-    int st = ensure_sort(c, 3, n, &sort, &records);
+    void* records = nullptr;
+    int st = ensure_sort(c, kSortSlots, c->surf[which], n, &sort, &records);
     if (st != TW_OK) return st;
     cudaEvent_t eb = nullptr, ee = nullptr;
     if (c->time_kernels) {
@@ -804,14 +833,14 @@ int tw_envelope_points(tw_ctx* c, const double* P, int64_t n, int which, uint8_t
     double* dP[kNumPipe];
     uint8_t* dO[kNumPipe];
     void* dS[kNumPipe];
-    bool records[kNumPipe];
+    void* records[kNumPipe];
     for (int k = 0; k < kNumPipe; ++k) {
         void* p;
         int st = ensure(c, k, 25 * (size_t)C + 256, &p);
         if (st != TW_OK) return st;
         dP[k] = (double*)p;
         dO[k] = (uint8_t*)p + 24 * (size_t)C;
-        st = ensure_sort(c, 3 + k, C, &dS[k], &records[k]);
+        st = ensure_sort(c, kSortSlots + k, c->surf[which], C, &dS[k], &records[k]);
         if (st != TW_OK) return st;
     }
     if (stage) {

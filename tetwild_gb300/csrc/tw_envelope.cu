@@ -1279,13 +1279,22 @@ size_t env_sort_scratch_bytes(int64_t n, int knob, bool records) {
            al(4 * (size_t)n + 4) + al(cub_scan_bytes(nbins)) + 256;
 }
 
+size_t env_record_bytes(int64_t n) { return sizeof(PointRec) * (size_t)n; }
+
 // Batches below this size are traversed in input order (sorting would cost
 // more than it saves).
 constexpr int64_t kSortMin = 4096;
 
+// The certified bulk test through the bins needs no more of a point than its
+// record; the other tests gather the binary64 coordinates.
+bool env_points_use_records(const Surface& S, int64_t n, double eps2, int precision, int knob) {
+    return precision == TW_PRECISION_FP32_CERTIFIED && knob != 0 && n >= kSortMin &&
+           n <= INT32_MAX && S.grid.boff && S.grid.eps2 == eps2;
+}
+
 void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2, uint8_t* out,
                        int precision, unsigned long long* counters, void* sort_scratch,
-                       int sort_knob, bool sort_records, int point_block, cudaStream_t s,
+                       int sort_knob, void* records, int point_block, cudaStream_t s,
                        cudaEvent_t ev_begin, cudaEvent_t ev_end) {
     if (n <= 0) return;
     const int block = 128;
@@ -1296,7 +1305,7 @@ void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2
     const EnvTree T = env_tree_for(S, eps2);
     const EpsParams E = eps_params(eps2);
     if (sort_scratch && n >= kSortMin && n <= INT32_MAX) {
-        SortLayout L = sort_layout(sort_scratch, n, sort_knob, sort_records);
+        SortLayout L = sort_layout(sort_scratch, n, sort_knob, records == sort_scratch);
         const unsigned nb = (unsigned)((n + 255) / 256);
         const int bits = sort_bits(n, sort_knob);
         if (T.boff && T.bid && sort_knob == 1 && (int64_t)T.nocc + 1 <= L.nbins) {
@@ -1330,11 +1339,9 @@ void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2
             size_t tb = L.temp_bytes;
             cub::DeviceScan::ExclusiveSum(L.temp, tb, L.count, (int)L.nbins, s);
         }
-        // the certified bulk test needs no more of a point than its record;
-        // the other tests gather the binary64 coordinates
-        if (L.rec && T.boff && precision == TW_PRECISION_FP32_CERTIFIED) {
-            k_point_place_rec<<<nb, 256, 0, s>>>(P, L.bin_rank, n, L.count, L.rec);
-            rec = L.rec;
+        if (records && env_points_use_records(S, n, eps2, precision, sort_knob)) {
+            rec = L.rec ? L.rec : static_cast<PointRec*>(records);
+            k_point_place_rec<<<nb, 256, 0, s>>>(P, L.bin_rank, n, L.count, rec);
         } else {
             k_point_place<<<nb, 256, 0, s>>>(L.bin_rank, n, L.count, L.idx);
             order = L.idx;

@@ -129,6 +129,9 @@ struct Surface {
 // point in place of the permutation (the certified test through the bin index
 // then reads the points in order; without it the points are gathered).
 size_t env_sort_scratch_bytes(int64_t n, int knob, bool records);
+// The records alone, and whether launch_env_points reads them for this batch.
+size_t env_record_bytes(int64_t n);
+bool env_points_use_records(const Surface& S, int64_t n, double eps2, int precision, int knob);
 
 // Device memory block owned by a context, grown on demand.
 struct Buffer {
@@ -171,7 +174,8 @@ struct tw_ctx {
     cudaEvent_t time_ev[2 * kTimeRing] = {};
     int sort_points = 1;     // Morton-order point queries (TW_TUNE_SORT_POINTS)
     int point_block = 384;   // threads per block of the certified grid test (TW_TUNE_POINT_BLOCK)
-    tw::Buffer scratch[10];
+    tw::Buffer scratch[13];
+    size_t records_refused = SIZE_MAX;   // least size of point records that did not fit
     // device counters, see the kCnt* indices below
     unsigned long long* counters = nullptr;
     // page-locked: word 0 receives the error word, word 1 an argument check's flag
@@ -272,13 +276,15 @@ void free_env_grid(tw_ctx* c, EnvGrid& G);
 // ---- launchers (tw_envelope.cu) ----
 // err: device word; bit 0 = traversal exceeded its bounds, bit 1 = a face
 // exceeded the per-row sample bound.
-// sort_scratch (env_sort_scratch_bytes(n, sort_knob, sort_records) bytes) enables
+// sort_scratch (env_sort_scratch_bytes(n, sort_knob, ...) bytes) enables
 // Morton-ordered traversal; with nullptr the points are traversed in input order.
+// records: env_record_bytes(n) bytes, or sort_scratch itself when that has room
+// for them, or nullptr.
 // precision: TW_PRECISION_FP64 or TW_PRECISION_FP32_CERTIFIED; counters is
 // the context's counter array (error word and statistics).
 void launch_env_points(const Surface& S, const double* P, int64_t n, double eps2, uint8_t* out,
                        int precision, unsigned long long* counters, void* sort_scratch,
-                       int sort_knob, bool sort_records, int point_block, cudaStream_t s,
+                       int sort_knob, void* records, int point_block, cudaStream_t s,
                        cudaEvent_t ev_begin = nullptr, cudaEvent_t ev_end = nullptr);
 void launch_env_faces(const Surface& S, const double* tris, int64_t n, double eps2, double sd,
                       uint8_t* out, int precision, unsigned long long* counters, cudaStream_t s);
