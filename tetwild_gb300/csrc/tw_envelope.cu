@@ -2427,9 +2427,11 @@ struct BuildScratch {
         return p;
     }
     void keep() { blocks.clear(); }
-    ~BuildScratch() {
+    void release() {
         for (auto& b : blocks) dev_free(c, b.first, b.second);
+        blocks.clear();
     }
+    ~BuildScratch() { release(); }
 };
 // Offsets of the parts of one allocation.
 struct Parts {
@@ -2549,8 +2551,17 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     bins = bins && suitable(hacc[2], hacc[3]);
     const int64_t nt = (int64_t)hacc[0], bt = bins ? (int64_t)hacc[2] : 0;
 
-    // what stays
-    BuildScratch K{c, {}};
+    // what stays; the bin index apart, which gives way to the grid where memory
+    // does not suffice for both (the call then ends with that error, the grid
+    // built and the bins left out)
+    BuildScratch K{c, {}}, KB{c, {}};
+    int st_bins = TW_OK;
+    auto drop_bins = [&]() {
+        st_bins = st;
+        st = TW_OK;
+        bins = false;
+        KB.release();
+    };
     const size_t list_bytes = 4 * (size_t)nt + 16, off_bytes = 4 * ((size_t)nmorton + 1),
                  ent_bytes = 4 * (size_t)(kFineWords + 1) * (size_t)bt, bid_bytes = 4 * (size_t)nmorton;
     int32_t* list = (int32_t*)K.get(list_bytes, st);
@@ -2558,47 +2569,50 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     uint32_t *boff = nullptr, *bent = nullptr;
     int32_t* bid = nullptr;
     if (bins) {
-        boff = (uint32_t*)K.get(off_bytes, st);
-        if (st == TW_OK) bent = (uint32_t*)K.get(ent_bytes, st);
-        if (st == TW_OK) bid = (int32_t*)K.get(bid_bytes, st);
-        if (st != TW_OK) return st;
+        boff = (uint32_t*)KB.get(off_bytes, st);
+        if (st == TW_OK) bent = (uint32_t*)KB.get(ent_bytes, st);
+        if (st == TW_OK) bid = (int32_t*)KB.get(bid_bytes, st);
+        if (st != TW_OK) drop_bins();
     }
     // the temporaries: the grid's (pairs twice, start) and the bins' (keys,
     // vals twice, leaves, masks, counts) follow one another in time
     int cell_bits = 0;
     while (cell_bits < 32 && (int64_t(1) << cell_bits) < n[0] * n[1] * n[2]) ++cell_bits;
-    size_t tb = 0, tbk = 0;
-    auto need = [&](size_t b) { tb = std::max(tb, b); };
+    size_t tb = 0, tb_bins = 0, tbk = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, tbk, (unsigned long long*)nullptr,
                                    (unsigned long long*)nullptr, (int)nt, 32, 32 + cell_bits, s);
-    need(tbk);
+    tb = std::max(tb, tbk);
     cub::DeviceRunLengthEncode::Encode(nullptr, tbk, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                        (uint32_t*)nullptr, (int*)nullptr, (int)nt, s);
-    need(tbk);
+    tb = std::max(tb, tbk);
     cub::DeviceScan::ExclusiveSum(nullptr, tbk, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nt, s);
-    need(tbk);
+    tb = std::max(tb, tbk);
     if (bins) {
         cub::DeviceRadixSort::SortPairs(nullptr, tbk, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                         (uint32_t*)nullptr, (uint32_t*)nullptr, (int)bt, 0,
                                         std::max(1, 3 * bits), s);
-        need(tbk);
+        tb_bins = std::max(tb_bins, tbk);
         cub::DeviceScan::ExclusiveSum(nullptr, tbk, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                       (int)(nmorton + 1), s);
-        need(tbk);
+        tb_bins = std::max(tb_bins, tbk);
         cub::DeviceScan::ExclusiveSum(nullptr, tbk, (int32_t*)nullptr, (int32_t*)nullptr,
                                       (int)nmorton, s);
-        need(tbk);
+        tb_bins = std::max(tb_bins, tbk);
     }
     Parts T;
-    const size_t o_temp = T.add(tb + 16), shared_at = T.at;
+    const size_t o_temp = T.add(tb + 16);
     const size_t o_pairs = T.add(8 * (size_t)nt), o_pairs2 = T.add(8 * (size_t)nt),
                  o_start = T.add(4 * (size_t)nt + 16);
     Parts TB;
-    TB.at = shared_at;
+    TB.add(tb_bins + 16);   // at o_temp too
     const size_t bb = 4 * (size_t)bt, o_k = TB.add(bb), o_k2 = TB.add(bb), o_v = TB.add(bb),
                  o_v2 = TB.add(bb), o_lf = TB.add(bb), o_m = TB.add(kFineWords * bb),
                  o_bc = TB.add(off_bytes);
     char* w = (char*)B.get(std::max(T.at, bins ? TB.at : 0), st);
+    if (st != TW_OK && bins) {
+        drop_bins();
+        w = (char*)B.get(T.at, st);
+    }
     if (st != TW_OK) return st;
     void* temp = w + o_temp;
 
@@ -2628,6 +2642,10 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     while ((1ULL << hbits) < 2ULL * (unsigned long long)nuniq) ++hbits;
     const size_t H = size_t(1) << hbits;
     uint4* slots = (uint4*)K.get(16 * H, st);
+    if (st != TW_OK && bins) {
+        drop_bins();
+        slots = (uint4*)K.get(16 * H, st);
+    }
     if (st != TW_OK) return st;
     cudaMemsetAsync(slots, 0xff, 16 * H, s);
     k_grid_insert<<<(unsigned)((nuniq + 255) / 256), 256, 0, s>>>(
@@ -2640,18 +2658,18 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
                  *bcnt = (uint32_t*)(w + o_bc);
         k_bin_cells<<<leaf_grid, kSatBlock, 0, s>>>(S.tri, nf, GB, bfoff, keys, vals, leaves);
         k_bin_masks<<<leaf_grid, kSatBlock, 0, s>>>(S.tri, nf, GF, bfoff, keys, masks);
-        t1 = tb;
+        t1 = tb_bins;
         cub::DeviceRadixSort::SortPairs(temp, t1, keys, keys2, vals, vals2, (int)bt, 0,
                                         std::max(1, 3 * bits), s);
         cudaMemsetAsync(bcnt, 0, off_bytes, s);
         k_bin_split<<<(unsigned)((bt + 255) / 256), 256, 0, s>>>(keys2, vals2, masks, leaves, bt,
                                                                  bent, bcnt);
-        t1 = tb;
+        t1 = tb_bins;
         cub::DeviceScan::ExclusiveSum(temp, t1, bcnt, boff, (int)(nmorton + 1), s);
         // the dense ids of the bins with entries, for the point sort
         const unsigned gm = (unsigned)((nmorton + 255) / 256);
         k_bin_flags<<<gm, 256, 0, s>>>(boff, nmorton, bid);
-        t1 = tb;
+        t1 = tb_bins;
         cub::DeviceScan::ExclusiveSum(temp, t1, bid, bid, (int)nmorton, s);
         k_bin_ids<<<gm, 256, 0, s>>>(boff, nmorton, bid, (int32_t*)(acc + 6));
     }
@@ -2660,6 +2678,7 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     if (e != cudaSuccess) return cuda_fail(c, e, "grid build");
     if ((hacc[5] & 0xffffffffULL) != 0) return TW_OK;
     K.keep();
+    KB.keep();
     EnvGrid& g = S.grid;
     for (int k = 0; k < 3; ++k) {
         g.lo[k] = lo[k];
@@ -2675,7 +2694,7 @@ int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaS
     g.slot_bytes = 16 * H;
     g.list_bytes = list_bytes;
     g.bin_factor = c->bin_cell;   // built for it, or found unsuitable
-    if (!bins) return TW_OK;
+    if (!bins) return st_bins;
     for (int k = 0; k < 3; ++k) {
         g.blo[k] = blo[k];
         g.bn[k] = (int32_t)bn[k];
