@@ -111,8 +111,10 @@ TW_API int tw_set_precision(tw_ctx* ctx, int mode);
 TW_API int tw_set_energy_form(tw_ctx* ctx, int form);
 typedef struct tw_stats {
     uint64_t exact_orientations;   /* orientation signs that needed the exact path */
-    uint64_t env_queries;          /* envelope points and face samples queried      */
-    uint64_t env_facet_tests;      /* facets reached by the traversals              */
+    uint64_t env_queries;          /* envelope points and face samples queried (not
+                                      the samples in a piece of a face that is known
+                                      to be inside as a whole)                      */
+    uint64_t env_facet_tests;      /* facets reached by these queries               */
     uint64_t env_facet_fp64;       /* of those, evaluated in binary64               */
     uint64_t amips_tets;           /* tets evaluated by the AMIPS kernels           */
     uint64_t amips_fp64;           /* of those, recomputed in binary64 (certified)  */

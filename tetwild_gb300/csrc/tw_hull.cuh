@@ -290,8 +290,7 @@ struct GridView {   // EnvTree's grid, passed by value
     const FacetCull* cull;
 };
 __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2in, float x0,
-                                                 float x1, float x2, uint32_t need,
-                                                 uint32_t* tests) {
+                                                 float x1, float x2, uint32_t need) {
     const uint32_t r1 = need & (need - 1u), r2 = r1 & (r1 - 1u);
     const int va = need ? __ffs(need) - 1 : 0, vb = r1 ? __ffs(r1) - 1 : 0, vc = r2 ? __ffs(r2) - 1 : 0;
     const float a[3] = {__shfl_sync(0xffffffffu, x0, va), __shfl_sync(0xffffffffu, x1, va),
@@ -305,7 +304,7 @@ __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2
     CertQuery q;
 #pragma unroll
     for (int k = 0; k < 3; ++k) q.ph[k] = y[k] = (a[k] + b[k] + c[k]) * 0.333333343f;
-    uint32_t i, e, n = 0;
+    uint32_t i, e;
     grid_cell_range(T, q, i, e);
     const uint32_t stride = (e - i + kDenseTries - 1) / kDenseTries;
     float best = e2in;
@@ -313,7 +312,6 @@ __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2
     for (; i < e; i += stride) {
         const int32_t lf = __ldg(T.glist + i);
         const float u = facet_upper(T.cull + lf, y, Mu2, best);
-        ++n;
         if (u < best) {
             best = u;
             leaf = lf;
@@ -325,9 +323,7 @@ __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2
 #pragma unroll
         for (int k = 0; k < 3; ++k) y[k] = v == 0 ? a[k] : v == 1 ? b[k] : c[k];
         in = facet_upper_in(T.cull + leaf, y, Mu2, e2in);
-        ++n;
     }
-    *tests = n;
     return in;
 }
 
@@ -341,7 +337,7 @@ __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2
 // taken (a face over many small facets: its pieces stay open).
 constexpr int kCutLeaves = 32;
 __device__ __forceinline__ bool pieces_inside(const EnvTree& T, const FaceFrame& h, bool vert,
-                                              const float* x, uint32_t need, TravStats& st) {
+                                              const float* x, uint32_t need) {
     uint32_t i = 0, e = 0;
     if (vert) {
         CertQuery q;
@@ -350,12 +346,9 @@ __device__ __forceinline__ bool pieces_inside(const EnvTree& T, const FaceFrame&
         grid_cell_range(T, q, i, e);
     }
     if (__reduce_max_sync(0xffffffffu, e - i) > (uint32_t)kDenseCell) {
-        uint32_t tests = 0;
         const GridView g{{T.glo[0], T.glo[1], T.glo[2]}, T.ginv, {T.gn[0], T.gn[1], T.gn[2]},
                          T.gshift, T.gmask, T.gslot, T.glist, T.cull};
-        const bool in = dense_pieces_inside(g, h.Mu2, h.e2in, x[0], x[1], x[2], need, &tests);
-        st.facets += tests;
-        return in;
+        return dense_pieces_inside(g, h.Mu2, h.e2in, x[0], x[1], x[2], need);
     }
     // the list is read one entry ahead of the leaf at hand
     uint32_t cur = i < e ? (uint32_t)__ldg(T.glist + i) : kNone;
@@ -377,7 +370,6 @@ __device__ __forceinline__ bool pieces_inside(const EnvTree& T, const FaceFrame&
         bool in = false;
         if (has) {
             in = facet_upper_in(T.cull + lf, x, Mu2, e2in);
-            ++st.facets;
             if (in) {
                 near1 = near0 == kNone ? near1 : near1 == kNone ? lf : near1;
                 near0 = near0 == kNone ? lf : near0;
@@ -422,10 +414,7 @@ __device__ __forceinline__ bool pieces_inside(const EnvTree& T, const FaceFrame&
         p[k] = __shfl_sync(0xffffffffu, x[k], vp);
         q[k] = __shfl_sync(0xffffffffu, x[k], vq);
     }
-    if (test) {
-        inside = crease_inside(T.cull + f, T.cull + g, o, p, q, Mu2, e2in);
-        st.facets += 4;
-    }
+    if (test) inside = crease_inside(T.cull + f, T.cull + g, o, p, q, Mu2, e2in);
     return inside;
 }
 
@@ -476,8 +465,8 @@ __device__ __forceinline__ bool vertex_out(const EnvTree& T, const EpsParams& E,
 // first open piece, and answers 1 when a vertex is certainly out.  2: open.
 // With KEEP the warps slice = 0 .. slices - 1 of a block may share the second
 // cuts, each writing its own cuts' pieces (the caller synchronises; open then
-// keeps cuts whose pieces are all inside, with open2 = 0).  nq counts the
-// pieces and vertices tested.
+// keeps cuts whose pieces are all inside, with open2 = 0).  st and nq count
+// the vertices tested, not the pieces (which are no samples).
 template <bool KEEP>
 __device__ __forceinline__ int hull_cut(const EnvTree& T, const EpsParams& E, const FaceFrame& h,
                                         const double* __restrict__ t, const CutTables& tab,
@@ -530,8 +519,7 @@ __device__ __forceinline__ int hull_cut(const EnvTree& T, const EpsParams& E, co
         float x[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) x[k] = fmaf(ra, h.d1[k], fmaf(rb, h.d2[k], h.p0[k]));
-        const bool ok = pieces_inside(T, h, vert, x, need, st);
-        if (need) ++nq;
+        const bool ok = pieces_inside(T, h, vert, x, need);
         const uint32_t bal = __ballot_sync(0xffffffffu, need && !ok);
         if (turn < 0) {
             open = bal;
