@@ -230,10 +230,11 @@ TW_API int tw_newton_stars_device(tw_ctx* ctx, const int32_t* star_off, const in
 /* Launch shape of the Newton step and the stages around it: block size (64,
  * 128, 256), stars in flight per block (8 to 32) and lanes per star of the
  * stages, TW_NEWTON_SHAPES in all; every shape gives bit-identical results.
- * tw_newton_autotune_device times every shape on the given batch (device
- * pointers, results written to out/moved), keeps the fastest in the context,
- * and reports it and, if ms_per_shape is non-NULL, each shape's time.  No
- * counterpart in the reference.                                            */
+ * tw_newton_autotune_device times the Newton step on the given batch (device
+ * pointers, results written to out/moved) for every block size and number of
+ * stars in flight, keeps the fastest in the context (with its lanes per star
+ * where a shape has both), and reports it and, if ms_per_shape is non-NULL,
+ * each shape's time.  No counterpart in the reference.                     */
 #define TW_NEWTON_SHAPES 10
 TW_API int tw_set_newton_shape(tw_ctx* ctx, int shape);
 TW_API int tw_newton_autotune_device(tw_ctx* ctx, const int32_t* star_off, const int32_t* tets,

@@ -1449,16 +1449,22 @@ int tw_set_newton_shape(tw_ctx* c, int shape) {
 }  // extern "C"
 
 namespace {
-// Times run(shape) for every launch shape (one untimed launch, then the best
-// of two timed ones, CUDA events on the context stream), keeps the fastest
-// shape in the context.
+// Times run(shape) for the launch shapes (one untimed launch, then the best of
+// two timed ones, CUDA events on the context stream), those that launch alike
+// once, and keeps the fastest in the context.  Among shapes alike it is the
+// context's own, or the one with its lanes per star: run did not time what
+// else they set (noise would choose).
 template <class Run>
-int autotune_shapes(tw_ctx* c, const char* where, int* best_shape, float* ms_per_shape, Run run) {
-    int best = c->newton_shape;
-    float best_ms = 0.0f;
+int autotune_shapes(tw_ctx* c, const char* where, bool stages, int* best_shape,
+                    float* ms_per_shape, Run run) {
+    const int own = c->newton_shape;
+    int best = 0;
+    float times[TW_NEWTON_SHAPES];
     for (int sh = 0; sh < newton_num_shapes(); ++sh) {
+        int twin = 0;
+        while (!newton_shapes_alike(twin, sh, stages)) ++twin;
         float ms = 0.0f;
-        for (int rep = 0; rep < 3; ++rep) {
+        for (int rep = 0; rep < 3 && twin == sh; ++rep) {
             cudaEventRecord(c->ev[3], c->stream);
             run(sh);
             cudaEventRecord(c->ev[4], c->stream);
@@ -1468,11 +1474,17 @@ int autotune_shapes(tw_ctx* c, const char* where, int* best_shape, float* ms_per
             cudaEventElapsedTime(&t, c->ev[3], c->ev[4]);
             if (rep == 1 || (rep == 2 && t < ms)) ms = t;
         }
-        if (ms_per_shape) ms_per_shape[sh] = ms;
-        if (sh == 0 || ms < best_ms) {
-            best_ms = ms;
-            best = sh;
-        }
+        times[sh] = twin == sh ? ms : times[twin];
+        if (ms_per_shape) ms_per_shape[sh] = times[sh];
+        if (times[sh] < times[best]) best = sh;
+    }
+    if (newton_shapes_alike(best, own, stages)) {
+        best = own;
+    } else {
+        for (int sh = newton_num_shapes() - 1; sh >= 0; --sh)
+            if (newton_shapes_alike(best, sh, stages) &&
+                newton_shape_group(sh) == newton_shape_group(own))
+                best = sh;
     }
     c->newton_shape = best;
     *best_shape = best;
@@ -1489,7 +1501,7 @@ int tw_newton_autotune_device(tw_ctx* c, const int32_t* star_off, const int32_t*
         return TW_ERR_ARG;
     if (!c->vx) return fail(c, TW_ERR_NO_MESH, "no resident mesh");
     Guard g(c->device);
-    return autotune_shapes(c, "tw_newton_autotune_device", best_shape, ms_per_shape, [&](int sh) {
+    return autotune_shapes(c, "tw_newton_autotune_device", false, best_shape, ms_per_shape, [&](int sh) {
         launch_newton_stars_shape(sh, c->precision, c->vx, c->vy, c->vz, star_off, tets, centers, nstars,
                                   c->newton_max_step, c->newton_max_it, out, moved, c->stream, c->energy_form);
     });
@@ -1512,7 +1524,7 @@ int tw_smooth_autotune_device(tw_ctx* c, const int32_t* star_off, const int32_t*
     int st = smooth_scratch(c, nstars, ntets, S);
     if (st != TW_OK) return st;
     const int keep = c->newton_shape;
-    st = autotune_shapes(c, "tw_smooth_autotune_device", best_shape, ms_per_shape, [&](int sh) {
+    st = autotune_shapes(c, "tw_smooth_autotune_device", true, best_shape, ms_per_shape, [&](int sh) {
         c->newton_shape = sh;
         smooth_launch(c, star_off, tets, face_flags, centers, kinds, nstars, any_surface, out,
                       status, S);

@@ -315,6 +315,10 @@ void launch_smooth_project(const Surface& Sin, const Surface& Sb, double eps2,
 // comparisons in binary32 where it can.  Every shape and precision gives
 // bit-identical results.
 int newton_num_shapes();
+// Lanes per star of a shape's stages, and whether two shapes launch the Newton
+// kernel, or a whole pass (stages), in the same way.
+int newton_shape_group(int shape);
+bool newton_shapes_alike(int a, int b, bool stages);
 void launch_newton_stars_shape(int shape, int precision, const double* vx, const double* vy,
                                const double* vz, const int32_t* star_off, const int32_t* tets,
                                const int32_t* centers, int32_t nstars, int max_step, int max_it,

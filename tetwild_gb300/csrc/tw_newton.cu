@@ -376,11 +376,24 @@ static int smooth_group(int shape, int* block) {
     return kNewtonShapes[shape].group;
 }
 
+static int wave_slots(int block, int group) { return std::min(kWaveSlots, 4 * block / group); }
+int newton_shape_group(int shape) {
+    int block;
+    return smooth_group(shape, &block);
+}
+// Of the ten shapes the Newton kernel has six configurations, 128 and 256
+// threads with 32 stars in flight three times each.
+bool newton_shapes_alike(int a, int b, bool stages) {
+    int ba, bb;
+    const int ga = smooth_group(a, &ba), gb = smooth_group(b, &bb);
+    return ba == bb && (stages ? ga == gb : wave_slots(ba, ga) == wave_slots(bb, gb));
+}
+
 template <bool SMOOTH, bool CERT>
 static void launch_wave(int shape, WaveArgs A, cudaStream_t s) {
     int block;
     const int group = smooth_group(shape, &block);
-    A.slots = std::min(kWaveSlots, 4 * block / group);
+    A.slots = wave_slots(block, group);
     // one star a block before two: the grid fills the SMs first
     const int grid = grid_for(A.nstars, 1, 512 / block);
     if (block == 64) k_newton_wave<SMOOTH, CERT, 64><<<grid, 64, 0, s>>>(A);
