@@ -101,7 +101,12 @@ TW_API int tw_memory_used(const tw_ctx* ctx, size_t* bytes);
  * in binary64 every query whose binary32 result falls inside a certified
  * error band (envelope: facets whose certified lower distance bound does not
  * exceed eps; AMIPS: tets whose certified relative error bound exceeds
- * 1e-5), so every decision equals the binary64 one.                         */
+ * 1e-5; Newton trials, smoothing and collapse qualities: comparisons that
+ * certified energy intervals leave open), so every decision equals the
+ * binary64 one.  TW_PRECISION_FP64 takes from certified binary32 bounds only
+ * what cannot change a result: signs of orientations, facets out of reach
+ * (points, face samples, nearest facets) and pieces of faces inside as a
+ * whole; every number is rounded as the binary64 operations round it.       */
 TW_API int tw_set_precision(tw_ctx* ctx, int mode);
 /* Energy form of every binary64 AMIPS evaluation of the context (the batch
  * calls, tet qualities, energy sweeps, Newton steps, smoothing passes and

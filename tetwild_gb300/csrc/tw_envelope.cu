@@ -1868,14 +1868,16 @@ __device__ __forceinline__ int face_prepare(const double* t, double sd, bool sha
 // the samples there.  (In one kernel the cut was held to the 16 warps per SM
 // of the sampling's 128 registers, and half of its stalls were barriers.)
 // Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
-// to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
-// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.1 and 0.25.
+// to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.8 ms
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.0 and 0.26.
 // Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
 constexpr int kFaceWarps = kFaceBlock / 32;
 constexpr int kCutBlocks = 8, kSampleBlocks = 4;   // blocks per SM
 constexpr uint8_t kFaceOpen = 2;
-// pieces that a sample is worth: its binary64 distance costs that of several
+// pieces of the second cut that a sample is worth, at most (300k certified faces:
+// 4.1-4.3 ms with 0.3, 2.05 with 0.6, 2.00 with 1.2; 20k binary64 faces: 0.345 ms
+// with 0.5, 0.262 with 1.0, 0.27-0.28 with 2.0)
 constexpr float kSampleCost32 = 0.6f, kSampleCost64 = 1.0f;
 
 // The warps take tiles of faces from a counter (faces over many small facets
@@ -1931,7 +1933,9 @@ __device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64
     flush_stats(st, counters, nq);
 }
 
-// Samples of a face from which on the block's warps share it.
+// Samples of a face from which on the block's warps share it (200k-star pass:
+// 10.3-10.8 ms with 128, 9.9 with 384, 9.9-10.1 with 1152; 20k binary64 faces:
+// 0.313, 0.262, 0.22).
 constexpr int kSharedFace = 384;
 
 // The open faces are sparse and their work differs by orders of magnitude
@@ -2473,7 +2477,7 @@ bool fit_grid(const Surface& S, double Rm, double cs, double step, Good good, fl
 // the cell or bin alone (the leaves are emitted in order and the radix sorts
 // are stable, so a cell's leaves stay ascending); the host waits three times
 // (the entry counts, the distinct cells, the end), and the temporaries are
-// two allocations: opening a 100k-facet surface took 19.1 ms, now 4.5.
+// two allocations: opening a 100k-facet surface took 19.3 ms, now 3.5.
 int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaStream_t s) {
     if (S.nf <= 0 || !(eps2 >= 0.0)) return TW_OK;
     if (S.grid.slot && S.grid.eps2 == eps2 && S.grid.cell_factor == cell_factor &&

@@ -277,9 +277,11 @@ __device__ __forceinline__ uint32_t common_leaf(uint32_t a0, uint32_t a1, uint32
 // nearest to its centroid, among up to kDenseTries of the centroid's cell
 // spread over the list, and its three vertices are tested against that one.
 // Out of line, its values passed singly: the common path keeps its registers.
-// 28: between 10 and 40 tries, the sum of both launches on 300k faces of the
-// lat-long sphere (up to 500 facets a cell at its poles) was least there (2.28
-// ms against 2.49 at 10, 2.29 at 40 and 2.63 without).
+// The call of 300k faces on the lat-long sphere (up to 500 facets a cell at its
+// poles; two runs, ms): kDenseCell 10 2.10-2.12, 28 2.03-2.06, 40 2.07-2.11, no
+// dense path 2.40-2.47; kDenseTries 8 2.08-2.16, 12 1.92-2.00, 24 2.03-2.06, 48
+// 2.18-2.32 (fewer tries leave more faces open, and the 200k-star pass at 9.9
+// either way).
 constexpr int kDenseCell = 28, kDenseTries = 24;
 struct GridView {   // EnvTree's grid, passed by value
     float glo[3], ginv;
@@ -334,7 +336,8 @@ __device__ __noinline__ bool dense_pieces_inside(GridView T, float Mu2, float e2
 // so the lanes merge their cells' ascending lists: each step takes the
 // smallest leaf left, and tests it, one record for the whole warp, when it is
 // listed for a vertex of a piece still open.  At most kCutLeaves leaves are
-// taken (a face over many small facets: its pieces stay open).
+// taken (a face over many small facets: its pieces stay open; 300k faces: 2.70
+// ms with 16, 2.05 with 32, 2.00-2.10 with 64).
 constexpr int kCutLeaves = 32;
 __device__ __forceinline__ bool pieces_inside(const EnvTree& T, const FaceFrame& h, bool vert,
                                               const float* x, uint32_t need) {
