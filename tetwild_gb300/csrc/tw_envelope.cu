@@ -1632,14 +1632,16 @@ __device__ __forceinline__ void face_query_box(const double* t, const FaceCtx& F
 
 #include "tw_hull.cuh"
 
+constexpr int kProbe = 1 << 20;   // 32 kProbe: more than the samples of a face's rim
 // The samples of one face with its header already computed, the whole warp:
 // 1 if some sample is out, 0 otherwise.  Samples in a cut known to be inside
 // (hull) are passed over; the others collect in the warp's queue (64 words of
 // shared memory, as rows_held) and are built and tested 32 at a time, so that the binary64
 // construction and the facet tests run on full warps.  slice / slices: the
 // warp takes every slices-th step of 32 samples; stop (shared, may be null):
-// set by another warp of the face that found a sample out.  Out of line: the
-// sampling kernel calls it from two places.
+// set by another warp of the face that found a sample out.  With slices = kProbe
+// the first 32 samples only.  Out of line: the sampling kernel calls it from two
+// places.
 template <bool FP32>
 __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
                                                     const double* __restrict__ tri,
@@ -1764,6 +1766,7 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
         if (drain(false, rim)) return 1;
     }
     if (drain(true, rim)) return 1;
+    if (slices == kProbe) return 0;
     // ...then the rows 1..M: those that meet an open cut are listed, and 32 at a
     // time each lane sets up one (start point and last index), the reference's
     // break (a row with distance(v0_m, v1_m) <= sd ends the rows) applies, and
@@ -1882,7 +1885,9 @@ constexpr float kSampleCost32 = 0.6f, kSampleCost64 = 1.0f;
 
 // The warps take tiles of faces from a counter (faces over many small facets
 // cost tens of times the others), an eighth of a warp's share each (4 to 32
-// faces), so that small batches spread over all SMs and large ones balance.
+// faces), so that small batches spread over all SMs and large ones balance; up
+// to a face a warp, one each (the call of 8 certified faces of 0.1 eps, 1.5 eps
+// out: 59 us with tiles of four, 46 so).
 template <bool FP32, class Ctx>
 __device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64_t n,
                                           unsigned long long* counters, Ctx ctx,
@@ -1894,7 +1899,7 @@ __device__ __forceinline__ void faces_cut(const double* __restrict__ tris, int64
     TravStats st;
     uint32_t nq = 0, nopen = 0;
     const int64_t warps = (int64_t)gridDim.x * kFaceWarps, share = n / (warps * 8);
-    const int tile = (int)(share < 4 ? 4 : share > 32 ? 32 : share);
+    const int tile = n <= warps ? 1 : (int)(share < 4 ? 4 : share > 32 ? 32 : share);
     for (;;) {
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(counters + kCntFaceCut, (unsigned long long)tile);
@@ -1944,10 +1949,14 @@ constexpr int kSharedFace = 384;
 // hold about a quarter of a block's share of the open ones (at most one a
 // thread); every thread prepares one of them, the warps take the small ones in
 // turn, and then the four warps share the samples and second cuts of each
-// large one (a launch otherwise lasts as long as its largest face).
+// large one (a launch otherwise lasts as long as its largest face).  A large
+// face that was not cut (its vertices not tested) is probed by one warp first:
+// one that is out ends there, where the four would have tested four times the
+// samples (8 binary64 faces of 40 sample spacings, 1.5 eps out, no grid: 0.90 ms,
+// with that and a block a face 0.32).  all: every face is open (no cutting launch ran).
 template <bool FP32, class Ctx>
 __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, int64_t n,
-                                             unsigned long long* counters, Ctx ctx,
+                                             unsigned long long* counters, Ctx ctx, bool all,
                                              uint8_t* __restrict__ out) {
     __shared__ CutTables tab;
     __shared__ FaceFrame frame[kFaceBlock];
@@ -1956,21 +1965,26 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
     __shared__ uint32_t queue[kFaceWarps][64];
     __shared__ int32_t rows_held[kFaceWarps][64];
     __shared__ uint16_t list[kFaceBlock];
-    __shared__ uint8_t small[kFaceBlock], large[kFaceBlock];
+    __shared__ uint8_t small[kFaceBlock], large[kFaceBlock], probe[kFaceBlock];
     __shared__ int held, nsmall, nlarge, next, found;
     __shared__ unsigned long long at;
-    const unsigned long long nopen = counters[kCntFaceOpen];
+    const unsigned long long nopen = all ? (unsigned long long)n : counters[kCntFaceOpen];
     if (nopen == 0) return;
-    fill_cut_tables(tab);
+    if (!all) fill_cut_tables(tab);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     TravStats st;
     uint32_t nq = 0;
     const int rot = (int)(blockIdx.x / ((gridDim.x + 3) / 4)) % kFaceWarps;
-    const double want = fmin(fmax((double)nopen / (4.0 * gridDim.x), 2.0), (double)kFaceBlock);
-    const int range = (int)fmin(want * ((double)n / (double)nopen), 4096.0) + 1;
-    for (;;) {
+    const bool few = nopen <= gridDim.x;
+    const double want = fmin(fmax((double)nopen / (4.0 * gridDim.x), few ? 1.0 : 2.0), (double)kFaceBlock);
+    const int range = (int)fmin(want * ((double)n / (double)nopen), 4096.0) + (few ? 0 : 1);
+    // a face a block: no counter (which the launch then leaves as it is)
+    const bool single = all && n <= (int64_t)gridDim.x;
+    for (bool first = true;; first = false) {
         if (threadIdx.x == 0)
-            at = atomicAdd(counters + kCntFaceNext, (unsigned long long)range);
+            at = !single ? atomicAdd(counters + kCntFaceNext, (unsigned long long)range)
+                 : first ? (unsigned long long)blockIdx.x
+                         : (unsigned long long)n;
         __syncthreads();
         const int64_t base = (int64_t)at;
         if (base >= n) break;
@@ -1986,7 +2000,7 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 // the others: all threads read, and stop before the list can overflow
                 const int step = min(kFaceBlock - before, faces - r0);
                 const int f = r0 + threadIdx.x;
-                if ((int)threadIdx.x < step && out[base + f] == kFaceOpen)
+                if ((int)threadIdx.x < step && (all || out[base + f] == kFaceOpen))
                     list[atomicAdd(&held, 1)] = (uint16_t)f;
                 r0 += step;
                 __syncthreads();
@@ -2010,10 +2024,11 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 const int state = face_prepare(t, sd, frame[mine].k2 >= 0, h, counters);
                 if (state != 2) {
                     out[f] = (uint8_t)state;
-                } else if (!h.trivial && h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace) {
-                    large[atomicAdd(&nlarge, 1)] = (uint8_t)mine;
                 } else {
-                    small[atomicAdd(&nsmall, 1)] = (uint8_t)mine;
+                    const bool big = !h.trivial && h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace;
+                    probe[mine] = big;
+                    if (big) large[atomicAdd(&nlarge, 1)] = (uint8_t)mine;
+                    if (!big || frame[mine].k2 < 0) small[atomicAdd(&nsmall, 1)] = (uint8_t)mine;
                 }
             }
             __syncthreads();
@@ -2024,6 +2039,7 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 if (j >= nsmall) break;
                 const int k = small[j];
                 const int64_t f = base + list[k];
+                const bool big = probe[k];
                 FaceCtx F;
                 double sd;
                 ctx(f, F, sd);
@@ -2031,18 +2047,23 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                     hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[warp], 0, 1, st, nq);
                 const uint8_t o =
                     env_face_samples<FP32>(head[k], tris + 9 * f, cuts[warp], frame[k].k2,
-                                           queue[warp], rows_held[warp], F, sd, 0, 1, nullptr, st,
-                                           nq);
-                if (lane == 0) out[f] = o;
+                                           queue[warp], rows_held[warp], F, sd, 0,
+                                           big ? kProbe : 1, nullptr, st, nq);
+                __syncwarp();
+                if (lane == 0) {
+                    out[f] = o;
+                    probe[k] = big && o;   // decided
+                }
                 __syncwarp();
             }
             for (int j = 0; j < nlarge; ++j) {
                 const int k = large[j];
                 const int64_t f = base + list[k];
+                __syncthreads();   // cuts[0] is free, found is 0, the probes are done
+                if (frame[k].k2 < 0 && probe[k]) continue;
                 FaceCtx F;
                 double sd;
                 ctx(f, F, sd);
-                __syncthreads();   // cuts[0] is free, found is 0
                 if (frame[k].k2 >= 0)
                     hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[0], warp,
                                    kFaceWarps, st, nq);
@@ -2087,9 +2108,9 @@ __global__ void __launch_bounds__(kFaceBlock, kCutBlocks)
 template <bool FP32>
 __global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
     k_env_faces(const double* __restrict__ tris, int64_t n,
-                const unsigned long long* __restrict__ n_dev, OneFaceCtx C,
+                const unsigned long long* __restrict__ n_dev, OneFaceCtx C, bool all,
                 uint8_t* __restrict__ out) {
-    faces_sample<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, out);
+    faces_sample<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, all, out);
 }
 
 // n_dev: nullptr, or the device count of the faces (at most n)
@@ -2097,16 +2118,19 @@ void launch_env_faces_dev(const Surface& S, const double* tris, const unsigned l
                           int64_t n, double eps2, double sd, uint8_t* out, int precision,
                           unsigned long long* counters, cudaStream_t s) {
     if (n <= 0) return;
+    // a surface without a grid cuts no face: the sampling launch takes them all
     const int block = kFaceBlock;
-    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
-    cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
+    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, 1, kSampleBlocks);
     const OneFaceCtx C{FaceCtx{env_tree_for(S, eps2), eps_params(eps2), counters}, sd};
+    const bool cut = C.F.T.gslot != nullptr;
+    if (cut || n_dev || n > gs)
+        cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
     if (precision == TW_PRECISION_FP32_CERTIFIED) {
-        k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
-        k_env_faces<true><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
+        if (cut) k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<true><<<gs, block, 0, s>>>(tris, n, n_dev, C, !cut, out);
     } else {
-        k_env_faces_cut<false><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
-        k_env_faces<false><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
+        if (cut) k_env_faces_cut<false><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<false><<<gs, block, 0, s>>>(tris, n, n_dev, C, !cut, out);
     }
 }
 
@@ -2198,7 +2222,7 @@ template <bool FP32>
 __global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
     k_env_faces_segs(const double* __restrict__ tris, int64_t n, SegFaceCtx C,
                      uint8_t* __restrict__ out) {
-    faces_sample<FP32>(tris, n, C.counters, C, out);
+    faces_sample<FP32>(tris, n, C.counters, C, false, out);
 }
 
 void launch_env_points_segs(const double* P, int64_t n, const void* segs, int nsegs, uint8_t* out,
@@ -2217,7 +2241,7 @@ void launch_env_faces_segs(const double* tris, int64_t n, const void* segs, int 
                            int precision, unsigned long long* counters, cudaStream_t s) {
     if (n <= 0 || nsegs <= 0) return;
     const int block = kFaceBlock;
-    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, kFaceWarps, kSampleBlocks);
+    const int gc = grid_for(n, kFaceWarps, kCutBlocks), gs = grid_for(n, 1, kSampleBlocks);
     cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
     const SegFaceCtx C{static_cast<const EnvSeg*>(segs), nsegs, counters};
     if (precision == TW_PRECISION_FP32_CERTIFIED) {
