@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -1647,14 +1648,19 @@ constexpr int kProbe = 1 << 20;   // 32 kProbe: more than the samples of a face'
 // set by another warp of the face that found a sample out.  With slices = kProbe
 // the first 32 samples only.  Out of line: the sampling kernel calls it from two
 // places.
-template <bool FP32>
+// !CUT: no part of the face is known to be inside (no hull, no queue): each step
+// of 32 samples is tested as it comes.
+template <bool FP32, bool CUT>
 __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
                                                     const double* __restrict__ tri,
                                                     const FaceCuts& hull, int k2, uint32_t* queue,
                                                     int32_t* rows_held,
-                                                    const FaceCtx& F, double sd, int slice,
+                                                    const FaceCtx& Fr, double sd, int slice,
                                                     int slices, const volatile int* stop,
                                                     TravStats& st, uint32_t& nq) {
+    // a copy keeps the tree's pointers in registers for the walk; the cut faces'
+    // tests through the grid are as fast without (and the registers short)
+    typename std::conditional<CUT, const FaceCtx&, const FaceCtx>::type F = Fr;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
     double tv[9];
@@ -1742,6 +1748,12 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
     const int NE = (h.M >= 1 && h.hasE) ? count_upto(h.NE, 1) : 0;
     const int NF = (h.M >= 1 && h.hasF) ? count_upto(h.NF, 1) : 0;
     const int NX = NA + 2 + NE + NF;
+    // !CUT: the lane's sample at once; true when one of the warp's is out
+    auto test = [&](bool have, const V3& p) -> bool {
+        const bool o = lane_out(have, p);
+        if (have) ++nq;
+        return __any_sync(0xffffffffu, o || (stop && *stop));
+    };
     auto rim = [&](bool have, uint32_t e) -> V3 {
         const int s = (int)e;
         if (!have) return fv.v0;
@@ -1753,6 +1765,10 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
     };
     for (int s0 = 32 * slice; s0 < NX; s0 += 32 * slices) {
         const int s = s0 + lane;
+        if (!CUT) {
+            if (test(s < NX, rim(s < NX, (uint32_t)s))) return 1;
+            continue;
+        }
         float x, y;   // the sample along v0->v1 and v0->v2
         if (s < NA) {
             x = (float)s * h.r01;
@@ -1770,7 +1786,7 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
         push(s < NX && !inside(x, y), (uint32_t)s);
         if (drain(false, rim)) return 1;
     }
-    if (drain(true, rim)) return 1;
+    if (CUT && drain(true, rim)) return 1;
     if (slices == kProbe) return 0;
     // ...then the rows 1..M: those that meet an open cut are listed, and 32 at a
     // time each lane sets up one (start point and last index), the reference's
@@ -1780,7 +1796,7 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
     // always listed: passing over rows never passes over a break.
     int held = 0;
     for (int base = 1; base <= h.M || held > 0; base += 32) {
-        if (base <= h.M) {
+        if (CUT && base <= h.M) {
             const int m = base + lane;
             const bool want = m <= h.M && (m + 1 >= h.M || hull_row_open(hull, k2, h.max_i,
                                                                          (float)m * h.rrow));
@@ -1790,14 +1806,17 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
             __syncwarp();
             if (held < 32 && base + 32 <= h.M) continue;
         }
-        const int batch = min(held, 32);
-        const int m = lane < batch ? rows_held[lane] : 0;
-        // what is left moves to the front (at most 31 entries)
-        held -= batch;
-        const int rest = lane < held ? rows_held[32 + lane] : 0;
-        __syncwarp();
-        if (lane < held) rows_held[lane] = rest;
-        __syncwarp();
+        const int batch = CUT ? min(held, 32) : min(h.M - base + 1, 32);
+        int m = base + lane;
+        if (CUT) {
+            m = lane < batch ? rows_held[lane] : 0;
+            // what is left moves to the front (at most 31 entries)
+            held -= batch;
+            const int rest = lane < held ? rows_held[32 + lane] : 0;
+            __syncwarp();
+            if (lane < held) rows_held[lane] = rest;
+            __syncwarp();
+        }
         V3 v{0.0, 0.0, 0.0};
         int N1 = -1;
         double dd = 0.0;
@@ -1842,12 +1861,17 @@ __device__ __noinline__ uint8_t env_face_samples(const SampleHeader& h,
                 if (c < 32 && ex <= s) r = c;
             }
             const int i = s - __shfl_sync(0xffffffffu, excl, r);
+            if (!CUT) {
+                if (test(s < total, in_row(s < total, ((uint32_t)r << 26) | (uint32_t)max(i, 0))))
+                    return 1;
+                continue;
+            }
             const float x = fmaf((float)i, h.r01, __shfl_sync(0xffffffffu, sx, r));
             const float y = __shfl_sync(0xffffffffu, sy, r);
             push(s < total && !inside(x, y), ((uint32_t)r << 26) | (uint32_t)i);
             if (drain(false, in_row)) return 1;
         }
-        if (drain(true, in_row)) return 1;
+        if (CUT && drain(true, in_row)) return 1;
         if (bal) break;
     }
     return 0;
@@ -1958,11 +1982,15 @@ constexpr int kSharedFace = 384;
 // face that was not cut (its vertices not tested) is probed by one warp first:
 // one that is out ends there, where the four would have tested four times the
 // samples (8 binary64 faces of 40 sample spacings, 1.5 eps out, no grid: 0.90 ms,
-// with that and a block a face 0.32).  all: every face is open (no cutting launch ran).
-template <bool FP32, class Ctx>
+// with that and a block a face 0.32).  !CUT: every face is open (no cutting launch
+// ran), and none is shared where each warp has one to itself, since each would walk
+// the tree for its candidate leaves; with the cut's queue and hull tests in its
+// place 54k such faces took 4.3 ms, 2.6 so (2.7 a face a warp in fixed blocks).
+template <bool FP32, bool CUT, class Ctx>
 __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, int64_t n,
-                                             unsigned long long* counters, Ctx ctx, bool all,
+                                             unsigned long long* counters, Ctx ctx,
                                              uint8_t* __restrict__ out) {
+    constexpr bool all = !CUT;
     __shared__ CutTables tab;
     __shared__ FaceFrame frame[kFaceBlock];
     __shared__ SampleHeader head[kFaceBlock];
@@ -1980,7 +2008,7 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
     TravStats st;
     uint32_t nq = 0;
     const int rot = (int)(blockIdx.x / ((gridDim.x + 3) / 4)) % kFaceWarps;
-    const bool few = nopen <= gridDim.x;
+    const bool few = nopen <= gridDim.x, share = !all || nopen <= (unsigned long long)kFaceWarps * gridDim.x;
     const double want = fmin(fmax((double)nopen / (4.0 * gridDim.x), few ? 1.0 : 2.0), (double)kFaceBlock);
     const int range = (int)fmin(want * ((double)n / (double)nopen), 4096.0) + (few ? 0 : 1);
     // a face a block: no counter (which the launch then leaves as it is)
@@ -2030,7 +2058,8 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 if (state != 2) {
                     out[f] = (uint8_t)state;
                 } else {
-                    const bool big = !h.trivial && h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace;
+                    const bool big = share && !h.trivial &&
+                                     h.N * (3.0 + 0.5 * (double)h.M) > (double)kSharedFace;
                     probe[mine] = big;
                     if (big) large[atomicAdd(&nlarge, 1)] = (uint8_t)mine;
                     if (!big || frame[mine].k2 < 0) small[atomicAdd(&nsmall, 1)] = (uint8_t)mine;
@@ -2048,10 +2077,10 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 FaceCtx F;
                 double sd;
                 ctx(f, F, sd);
-                if (frame[k].k2 >= 0)
+                if (CUT && frame[k].k2 >= 0)
                     hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[warp], 0, 1, st, nq);
                 const uint8_t o =
-                    env_face_samples<FP32>(head[k], tris + 9 * f, cuts[warp], frame[k].k2,
+                    env_face_samples<FP32, CUT>(head[k], tris + 9 * f, cuts[warp], frame[k].k2,
                                            queue[warp], rows_held[warp], F, sd, 0,
                                            big ? kProbe : 1, nullptr, st, nq);
                 __syncwarp();
@@ -2069,11 +2098,11 @@ __device__ __forceinline__ void faces_sample(const double* __restrict__ tris, in
                 FaceCtx F;
                 double sd;
                 ctx(f, F, sd);
-                if (frame[k].k2 >= 0)
+                if (CUT && frame[k].k2 >= 0)
                     hull_cut<true>(F.T, F.E, frame[k], tris + 9 * f, tab, &cuts[0], warp,
                                    kFaceWarps, st, nq);
                 __syncthreads();
-                if (env_face_samples<FP32>(head[k], tris + 9 * f, cuts[0], frame[k].k2,
+                if (env_face_samples<FP32, CUT>(head[k], tris + 9 * f, cuts[0], frame[k].k2,
                                            queue[warp], rows_held[warp], F, sd, warp, kFaceWarps,
                                            &found, st, nq))
                     found = 1;
@@ -2110,12 +2139,12 @@ __global__ void __launch_bounds__(kFaceBlock, kCutBlocks)
                     uint8_t* __restrict__ out) {
     faces_cut<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, out);
 }
-template <bool FP32>
+template <bool FP32, bool CUT>
 __global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
     k_env_faces(const double* __restrict__ tris, int64_t n,
-                const unsigned long long* __restrict__ n_dev, OneFaceCtx C, bool all,
+                const unsigned long long* __restrict__ n_dev, OneFaceCtx C,
                 uint8_t* __restrict__ out) {
-    faces_sample<FP32>(tris, faces_count(n, n_dev), C.F.counters, C, all, out);
+    faces_sample<FP32, CUT>(tris, faces_count(n, n_dev), C.F.counters, C, out);
 }
 
 // n_dev: nullptr, or the device count of the faces (at most n)
@@ -2130,12 +2159,16 @@ void launch_env_faces_dev(const Surface& S, const double* tris, const unsigned l
     const bool cut = C.F.T.gslot != nullptr;
     if (cut || n_dev || n > gs)
         cudaMemsetAsync(counters + kCntFaceOpen, 0, 3 * sizeof(unsigned long long), s);
-    if (precision == TW_PRECISION_FP32_CERTIFIED) {
-        if (cut) k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
-        k_env_faces<true><<<gs, block, 0, s>>>(tris, n, n_dev, C, !cut, out);
+    const bool cert = precision == TW_PRECISION_FP32_CERTIFIED;
+    if (!cut) {
+        auto kernel = cert ? k_env_faces<true, false> : k_env_faces<false, false>;
+        kernel<<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
+    } else if (cert) {
+        k_env_faces_cut<true><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<true, true><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
     } else {
-        if (cut) k_env_faces_cut<false><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
-        k_env_faces<false><<<gs, block, 0, s>>>(tris, n, n_dev, C, !cut, out);
+        k_env_faces_cut<false><<<gc, block, 0, s>>>(tris, n, n_dev, C, out);
+        k_env_faces<false, true><<<gs, block, 0, s>>>(tris, n, n_dev, C, out);
     }
 }
 
@@ -2227,7 +2260,7 @@ template <bool FP32>
 __global__ void __launch_bounds__(kFaceBlock, kSampleBlocks)
     k_env_faces_segs(const double* __restrict__ tris, int64_t n, SegFaceCtx C,
                      uint8_t* __restrict__ out) {
-    faces_sample<FP32>(tris, n, C.counters, C, false, out);
+    faces_sample<FP32, true>(tris, n, C.counters, C, out);
 }
 
 void launch_env_points_segs(const double* P, int64_t n, const void* segs, int nsegs, uint8_t* out,
