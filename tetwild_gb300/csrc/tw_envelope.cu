@@ -865,7 +865,7 @@ __device__ __forceinline__ bool sat_cell(const SatLeaf& l, const SatSlab* slab, 
 // leaf's count and the total; a leaf whose box spans more than limit cells
 // marks the grid unsuitable (*too_big), and the counts, which nothing then
 // reads, are left there (uploading 3k facets of all sizes: 1.62 ms without that,
-// 0.43 so; 1.25 with a warp a leaf).  Filling: each leaf's cells from
+// 0.50 so; 1.25 with a warp a leaf).  Filling: each leaf's cells from
 // foff[leaf] on, in box order (fill(at, leaf, x, y, z), one lane each).
 template <class Fill>
 __device__ __forceinline__ void sat_cells(const double* __restrict__ tri, int32_t nf,
@@ -898,7 +898,7 @@ __device__ __forceinline__ void sat_cells(const double* __restrict__ tri, int32_
         uint32_t at = fcnt ? 0u : __ldg(foff + f0 + k);
         const uint32_t end = fcnt ? 0xffffffffu : __ldg(foff + f0 + k + 1);
         for (int q0 = 0; q0 < nbox; q0 += 32) {
-            if (too_big && (q0 & 1023) == 0 &&
+            if (too_big && q0 && (q0 & 1023) == 0 &&   // long boxes only: a load each
                 __shfl_sync(0xffffffffu, *(volatile const int*)too_big, 0))
                 return;
             int x = 0, y = 0, z = 0;
