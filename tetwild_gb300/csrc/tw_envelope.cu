@@ -1899,9 +1899,9 @@ __device__ __forceinline__ int face_prepare(const double* t, double sd, bool sha
 // face by a warp, which cuts it again, now keeping its open pieces, and tests
 // the samples there.  (In one kernel the cut was held to the 16 warps per SM
 // of the sampling's 128 registers, and half of its stalls were barriers.)
-// Sampling every face in full, as before: 12.0 ms for 300k faces (edges 4e-3
-// to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.8 ms
-// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.0 and 0.26.
+// Sampling every face in full, as before: 12.4 ms for 300k faces (edges 4e-3
+// to 3e-2, eps 1e-3, spacing eps / 2, 100k-facet sphere, certified) and 2.7 ms
+// for 20k (edges 0.02 to 0.17, spacing 2.4 eps, binary64); now 2.0 and 0.25.
 // Ctx(f, F, sd) gives face f's tree, eps and sampling distance.
 constexpr int kFaceBlock = 128;
 constexpr int kFaceWarps = kFaceBlock / 32;
@@ -2539,7 +2539,7 @@ bool fit_grid(const Surface& S, double Rm, double cs, double step, Good good, fl
 // the cell or bin alone (the leaves are emitted in order and the radix sorts
 // are stable, so a cell's leaves stay ascending); the host waits three times
 // (the entry counts, the distinct cells, the end), and the temporaries are
-// two allocations: opening a 100k-facet surface took 19.3 ms, now 3.5.
+// two allocations: opening a 100k-facet surface took 19.4 ms, now 3.5.
 int build_env_grid(tw_ctx* c, Surface& S, double eps2, double cell_factor, cudaStream_t s) {
     if (S.nf <= 0 || !(eps2 >= 0.0)) return TW_OK;
     if (S.grid.slot && S.grid.eps2 == eps2 && S.grid.cell_factor == cell_factor &&
